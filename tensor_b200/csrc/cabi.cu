@@ -277,6 +277,8 @@ int32_t tb200_gguf_device_status(uint32_t* status, TensorErrorV1* error) {
   if ((e = read_gemv_status(&a, true)) != cudaSuccess) return cuda_fail(error, "reading GEMV status", e);
   if (!a) a = t;
   if ((e = read_gemm_status(&b, true)) != cudaSuccess) return cuda_fail(error, "reading GEMM status", e);
+  if ((e = read_gemm_pair_status(&t, true)) != cudaSuccess) return cuda_fail(error, "reading GEMM status", e);
+  if (!b) b = t;
   if ((e = read_barrier_status(&c, true)) != cudaSuccess) return cuda_fail(error, "reading barrier status", e);
   if (status) *status = a ? a : (b ? b : c);
   if (a || b || c)
@@ -807,8 +809,14 @@ int32_t gemm_common(int32_t format, int32_t x_dtype, const void* x, const void* 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint8_t* wp = static_cast<const uint8_t*>(w);
   if (variant != TB200_VARIANT_SIMPLE) {
+    const char* detail = "";
+    if (!sched) sched = lookup_schedule(kOpGemm, format, m, n, k);
+    if ((!sched || !sched->gemm_shape) && gemm_pair_supported(format, m, n, k, *dev)) {
+      cudaError_t e = launch_gemm_pair(format, x, wp, out, m, n, k, st, &detail);
+      if (e != cudaSuccess) return cuda_fail(error, *detail ? detail : "tcgen05 GEMM launch", e);
+      return ok(error);
+    }
     if (gemm_fast_supported(format, m, n, k, *dev)) {
-      const char* detail = "";
       if (sched && !gemm_shape_legal(sched->gemm_shape, m, *dev))
         return fail(error, TENSOR_ERROR_ARGUMENT, "GEMM shape %d is not legal on this device", sched->gemm_shape);
       cudaError_t e = launch_gemm_fast(format, x, wp, out, m, n, k, st, &detail, sched);

@@ -198,6 +198,12 @@ cudaError_t launch_gemm_fast(int fmt, const void* x, const uint8_t* w, float* ou
                              const Schedule* sched = nullptr);
 bool gemm_shape_legal(int shape, long long m, const DeviceInfo& dev);
 
+// The same GEMM for all four formats on pairs of CTAs (gemm_pair.cu): what the entry points run unless a schedule pins
+// one of the shapes above.
+bool gemm_pair_supported(int fmt, long long m, long long n, long long k, const DeviceInfo& dev);
+cudaError_t launch_gemm_pair(int fmt, const void* x, const uint8_t* w, float* out, long long m, long long n, long long k,
+                             cudaStream_t stream, const char** detail);
+
 // 2-D tiled TMA tensor map (128 bytes, 64-byte aligned) over a row-major matrix; elements are bf16
 // or opaque 8-byte words.  Returns false if the driver entry point is unavailable or rejects it.
 enum class TmaType { kBF16, kU64 };
@@ -212,6 +218,7 @@ bool allocation_range(const void* ptr, void** base, size_t* size);
 cudaError_t read_gemv_status(unsigned int* value, bool clear);
 cudaError_t read_gemv_tc_status(unsigned int* value, bool clear);
 cudaError_t read_gemm_status(unsigned int* value, bool clear);
+cudaError_t read_gemm_pair_status(unsigned int* value, bool clear);
 cudaError_t read_barrier_status(unsigned int* value, bool clear);
 
 }  // namespace tb200

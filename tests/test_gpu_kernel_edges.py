@@ -41,3 +41,41 @@ def test_dequant_partial_units_and_two_byte_alignment(name, offset):
         tb.dequantize(buf[offset:offset + raw.size], name, n, k, out=out)
         want = oracle.dequantize(raw, name, n, k)
         assert np.array_equal(out.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
+# ---- prefill GEMM: pairs of CTAs, 256 weight rows x 32 .. 256 tokens, 64-wide k-blocks, K split over 1, 2 or 4 pairs --
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("m,n,blocks", [
+    (1, 1, 1), (17, 127, 3), (32, 257, 5), (33, 300, 8), (64, 256, 16), (130, 129, 9), (256, 513, 7), (257, 384, 12),
+    (300, 1031, 17), (513, 260, 24),
+])
+def test_gemm_pair_edges(name, m, n, blocks):
+    # blocks counts 256 weights for the K-quants and 32 for the others: k-blocks and raw chunks with every remainder,
+    # rows of every 2-byte alignment
+    k = blocks * tb.get_format(name).weights * (1 if tb.get_format(name).weights == 256 else 5)
+    raw = oracle.make_weights(name, n, k, seed=n + k)
+    x = oracle.make_activations(m, k, seed=m, dtype="bf16")
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gemm(to_dev(x, torch.bfloat16), to_dev(raw), name, n, k, out=out)
+    want = oracle.gemm_ref(x, raw, name, n, k, operand="bf16")
+    # bf16 operands are the same bits on both sides; fp32 sums of K <= 6144 products of random sign differ by a few
+    # times sqrt(K) 2^-24 = 4.7e-6 of the result
+    assert oracle.rel_frobenius(out.cpu().numpy(), want) < 2e-5
+
+
+@pytest.mark.parametrize("name,m,n,k", [("q4_k", 600, 12300, 512), ("q6_k", 600, 12300, 768), ("q6_k", 520, 17000, 256),
+                                        ("q8_0", 700, 11000, 544), ("q4_0", 700, 11000, 352)])
+def test_gemm_pair_several_tiles_per_pair(name, m, n, k):
+    """More tiles than pairs: accumulator sets, stages and raw chunks go round."""
+    raw = oracle.make_weights(name, n, k, seed=3)
+    x = oracle.make_activations(m, k, seed=4, dtype="bf16")
+    xd, wd = to_dev(x, torch.bfloat16), to_dev(raw)
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gemm(xd, wd, name, n, k, out=out)
+    w = tb.dequantize(wd, name, n, k).to(torch.bfloat16).double()
+    want = xd.double() @ w.t()
+    assert float((out.double() - want).norm() / want.norm()) < 2e-5  # as above
+    again = torch.full((m, n), float("nan"), device=dev())
+    tb.gemm(xd, wd, name, n, k, out=again)
+    assert torch.equal(out, again)
