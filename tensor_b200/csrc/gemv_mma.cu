@@ -1283,7 +1283,8 @@ GemvPlan plan_gemv_fast(int fmt, int xt, long long m, long long n, long long k,
       const int per = (nsb + splits - 1) / splits;
       if ((splits - 1) * per >= nsb) continue;  // an empty K range
       const long long need =
-          splits > 1 ? (kCounterBytes + (long long)splits * m * n * 4) : 0;
+          // (whole 256 bytes: the converted activations behind it move in 16-byte units, and m n may be odd)
+          splits > 1 ? (kCounterBytes + (long long)splits * m * n * 4 + 255) / 256 * 256 : 0;
       if (need > scratch_bytes_available) continue;
       int stages = 0, red_bufs = 2;
       const int warps = choose_warps(per, per_sm == 1 ? kMaxConsumerWarps : kNarrowWarps);

@@ -79,3 +79,14 @@ def test_gemm_pair_several_tiles_per_pair(name, m, n, k):
     again = torch.full((m, n), float("nan"), device=dev())
     tb.gemm(xd, wd, name, n, k, out=again)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 777, 4352), (3, 257, 18944), (15, 129, 12288)])
+def test_split_gemv_with_odd_row_counts(m, n, k):
+    """K split over CTAs with an odd number of partial sums: what lies behind them in the scratch stays aligned."""
+    raw = oracle.make_weights("q4_k", n, k, seed=61)
+    x = oracle.make_activations(m, k, seed=62, dtype="bf16")
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gguf(m, n, k, "q4_k", variant="fast").launch(to_dev(x, torch.bfloat16), to_dev(raw), out)
+    assert oracle.rel_frobenius(out.cpu().numpy(), oracle.gemv_ref(x, raw, "q4_k", n, k)) < 2e-5
+    assert tb.device_status() == 0

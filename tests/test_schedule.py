@@ -108,3 +108,10 @@ def test_measured_search_behind_the_parity_gate(op, name, m, n, k):
     finally:
         schedule.clear()
     assert tb.device_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(9, 777, 4352), (3, 257, 18944), (15, 129, 12288), (2, 1031, 28672)])
+def test_scratch_regions_of_a_split_plan_are_aligned(m, n, k):
+    """The converted activations lie behind splits x m x n partial sums and move in 16-byte units."""
+    plan = tb.gemv_plan("q4_k", m, n, k)
+    assert plan["k_splits"] > 1 and plan["scratch_bytes"] % 256 == 0
