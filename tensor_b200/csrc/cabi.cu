@@ -303,6 +303,20 @@ int32_t tb200_gguf_dequant(int32_t format, const void* w, float* out, int64_t n,
 }  // extern "C"
 
 namespace {
+// Whether the default entry points run a decode GEMV on the kernel that keeps the activations in registers.
+bool use_frag(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k, int32_t variant, int out_count,
+              const PeerSync* peers, const Schedule* sched) {
+  if (variant != TB200_VARIANT_AUTO || out_count != 1 || (peers && peers->flags) || sched) return false;
+  if (!gemv_frag_supported(format, x_dtype, m, n, k)) return false;
+  // Where another kernel is ahead (us on B200, this one | that one): batch 1 on the integer dot-product units (Q6_K
+  // 4096 x 12288 19.8 | 13.7, Q8_0 12288 x 4096 19.4 | 12.4, Q4_0 13.8 | 9.7) and Q4_K's own pipeline with 2-byte
+  // activations (18944 x 3584: batch 1 17.7 | 10.9, batch 16 23.8 | 19.7).  Ahead here: Q6_K 4096 x 12288 at batch 16
+  // 27.6 | 46.5 (tensor memory), Q8_0 and Q4_0 12288 x 4096 at batch 8 19.8 | 132 and 14.7 | 102 (SIMT).
+  if (gemv_dp4a_supported(format, x_dtype, m, n, k)) return false;
+  if (format == kQ4_K && x_dtype != kF32) return false;
+  return !lookup_schedule(kOpGemv, format, m, n, k);  // a schedule recorded for the shape names the kernel it was searched on
+}
+
 // Shared by the plain and the sharded entry points: `out` says where the [m, n] result goes.
 int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* w, const OutSpec& out, int64_t m,
                     int64_t n, int64_t k, void* scratch, int64_t scratch_bytes, int32_t variant, void* stream,
@@ -318,6 +332,12 @@ int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* 
   if (int32_t s = require_device(error, &dev)) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint8_t* wp = static_cast<const uint8_t*>(w);
+  if (use_frag(format, x_dtype, m, n, k, variant, out.count, peers, sched)) {
+    if (prep_mode == kPrepOnly) return ok(error);  // (it converts the activations itself)
+    cudaError_t e = launch_gemv_frag(format, x_dtype, x, wp, out, m, n, k, st);
+    if (e == cudaSuccess) return ok(error);
+    if (e != cudaErrorInvalidValue) return cuda_fail(error, "decode GEMV launch", e);
+  }
   if (prep_mode == kPrepOnly) {
     // only the conversion launch of the pipelined kernel, where this call would take that kernel and its plan
     // converts ahead (the same conditions as below lead there)
@@ -548,6 +568,14 @@ int32_t tb200_gguf_gemv_pair(int32_t format, int32_t x_dtype, const void* x, con
         return ok(error);
       }
     }
+    if (n1 % kGemvTileRows == 0 && use_frag(format, x_dtype, m, n, k, variant, 1, nullptr, nullptr)) {
+      OutSpec both = single_output(out, n);
+      both.ptr2[0] = out + n1;
+      cudaError_t e = launch_gemv_frag(format, x_dtype, x, static_cast<const uint8_t*>(w1), both, m, n, k,
+                                       static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(w2), n1);
+      if (e == cudaSuccess) return ok(error);
+      if (e != cudaErrorInvalidValue) return cuda_fail(error, "decode GEMV launch (two weights)", e);
+    }
     GemvPlan plan = plan_gemv_fast(format, x_dtype, m, n, k, scratch ? scratch_bytes : 0, *dev);
     if (plan.supported && plan.k_splits == 1 && n1 % kGemvTileRows == 0) {
       OutSpec both = single_output(out, n);
@@ -631,6 +659,16 @@ static int32_t gemv_pair_sharded_impl(int32_t format, int32_t x_dtype, const voi
         if (e != cudaSuccess) return cuda_fail(error, "tensor-memory GEMV launch (two weights, sharded)", e);
         return ok(error);
       }
+    }
+    if (n1 % kGemvTileRows == 0 &&
+        use_frag(format, x_dtype, m, n, k, variant, out_count, peers.flags ? &peers : nullptr, nullptr)) {
+      if (prep_mode == kPrepOnly) return ok(error);
+      OutSpec both = single_output(outs1[0] + col_offset1, out_ld);
+      both.ptr2[0] = outs2[0] + col_offset2;
+      cudaError_t e = launch_gemv_frag(format, x_dtype, x, static_cast<const uint8_t*>(w1), both, m, n, k,
+                                       static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(w2), n1);
+      if (e == cudaSuccess) return ok(error);
+      if (e != cudaErrorInvalidValue) return cuda_fail(error, "decode GEMV launch (two weights)", e);
     }
     GemvPlan plan = plan_gemv_fast(format, x_dtype, m, n, k, scratch ? scratch_bytes : 0, *dev);
     if (plan.supported && plan.k_splits == 1 && n1 % kGemvTileRows == 0) {
@@ -899,8 +937,13 @@ ListUnits list_units(const TB200GemvItem* items, int count, const TcLaunchItem* 
       // a tile boundary); otherwise they are two units with a slice each
       const GemvPlan both = plan_gemv_fast(items[i].format, kBF16, items[i].m, items[i].n + items[i + 1].n, items[i].k,
                                            (long long)1 << 40, dev);
-      pair = both.supported && both.k_splits == 1 && items[i].n % kGemvTileRows == 0;
-      if (pair) need = both.scratch_bytes;
+      const bool pipelined = both.supported && both.k_splits == 1 && items[i].n % kGemvTileRows == 0;
+      pair = pipelined || (items[i].n % kGemvTileRows == 0 &&
+                           use_frag(items[i].format, items[i].x_dtype, items[i].m, items[i].n + items[i + 1].n, items[i].k,
+                                    variant, items[i].out_count, nullptr, nullptr));
+      if (pipelined) need = both.scratch_bytes;
+      else if (pair)
+        need = std::max<long long>(need, tb200_gguf_gemv_scratch_bytes(items[i].format, items[i + 1].m, items[i + 1].n, items[i + 1].k));
     }
     need = (need + 255) / 256 * 256;
     u.first[u.count] = i;
@@ -1002,7 +1045,7 @@ int32_t tb200_gguf_gemv_list(const TB200GemvItem* items, int32_t count, void* sc
     }
     PeerSync first = peers;  // ... and ONE launch runs them, after waiting for the peers like the first GEMV
     first.flags = wait_flag;
-    cudaError_t e = launch_gemv_prepare_jobs(conversions, wait_flag ? &first : nullptr, st);
+    cudaError_t e = !conversions.count ? cudaSuccess : launch_gemv_prepare_jobs(conversions, wait_flag ? &first : nullptr, st);
     if (e != cudaSuccess) return cuda_fail(error, "activation conversion launch (list)", e);
   }
   long long offset = 0;

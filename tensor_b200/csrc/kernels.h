@@ -165,6 +165,12 @@ bool gemv_dp4a_supported(int fmt, int xt, long long m, long long n, long long k)
 cudaError_t launch_gemv_dp4a(int fmt, int xt, const void* x, const uint8_t* w, const OutSpec& out, long long n,
                              long long k, cudaStream_t stream, const PeerSync* peers = nullptr);
 
+// Any format, activation type and row alignment at m <= 16, activations in registers (gemv_frag.cu): one destination, no
+// scratch.  w2, n1: a grouped launch whose rows from n1 on (a multiple of kGemvTileRows) come from a second weight.
+bool gemv_frag_supported(int fmt, int xt, long long m, long long n, long long k);
+cudaError_t launch_gemv_frag(int fmt, int xt, const void* x, const uint8_t* w, const OutSpec& out, long long m, long long n,
+                             long long k, cudaStream_t stream, const uint8_t* w2 = nullptr, long long n1 = 0);
+
 bool gemv_tc_supported(int fmt, int xt, long long m, long long n, long long k);
 // Scratch a list needs (arrival counters, partial sums of row tiles that span CTAs, converted
 // activations); zero before the first use, 256-byte aligned.

@@ -90,3 +90,48 @@ def test_split_gemv_with_odd_row_counts(m, n, k):
     tb.gguf(m, n, k, "q4_k", variant="fast").launch(to_dev(x, torch.bfloat16), to_dev(raw), out)
     assert oracle.rel_frobenius(out.cpu().numpy(), oracle.gemv_ref(x, raw, "q4_k", n, k)) < 2e-5
     assert tb.device_status() == 0
+
+
+# ---- decode GEMV with activations in registers: slices of 256, 16 slices a CTA, clusters along K, tiles of 16 rows ----
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("m,n,blocks,x", [
+    (2, 1, 1, "bf16"), (3, 15, 2, "f16"), (8, 17, 9, "bf16"), (9, 100, 5, "bf16"), (16, 2500, 3, "f16"), (16, 33, 17, "bf16"),
+    (5, 513, 33, "bf16"), (7, 20, 112, "bf16"), (1, 31, 16, "f32"), (2, 300, 7, "f32"), (3, 49, 40, "f32"), (16, 64, 11, "f32"),
+    (1, 130, 15, "bf16"),
+])
+def test_gemv_frag_edges(name, m, n, blocks, x):
+    # blocks counts 256 weights for the K-quants and 32 for the others (times 5 where that leaves a part of a slice)
+    step = tb.get_format(name).weights
+    k = blocks * step if step == 256 else blocks * step * 5
+    raw = oracle.make_weights(name, n, k, seed=n + k)
+    xs = oracle.make_activations(m, k, seed=m, dtype="f32" if x == "f32" else x)
+    dtype = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[x]
+    xd, wd = to_dev(xs, dtype), to_dev(raw)
+    kernel = tb.gguf(m, n, k, name, x_dtype=dtype)
+    out, again = (torch.full((m, n), float("nan"), device=dev()) for _ in range(2))
+    kernel.launch(xd, wd, out)
+    kernel.launch(xd, wd, again)
+    assert torch.equal(out, again)
+    want = xd.double() @ tb.dequantize(wd, name, n, k).double().t()
+    # exact operands; fp32 sums of up to 28672 products: a few times sqrt(K) 2^-24 = 1e-5 (Q4_K's own pipeline, which
+    # takes its 2-byte activations, loses three bits to the offset of its integers)
+    assert float((out.double() - want).norm() / want.norm()) < (2e-5 if name == "q4_k" else 1e-5)
+
+
+@pytest.mark.parametrize("name", ["q8_0", "q4_0", "q6_k"])
+def test_gemv_frag_special_values(name):
+    """Rows with an infinity or a NaN stay with themselves; zero and tiny rows keep their scale."""
+    n, k = 40, 512
+    wd = to_dev(oracle.make_weights(name, n, k, seed=5))
+    x = torch.randn(5, k, device=dev(), generator=torch.Generator(device=dev()).manual_seed(1)).to(torch.bfloat16)
+    x[0] = 0
+    x[1] *= 2.0 ** -100
+    x[2, 7] = float("nan")
+    x[3, 9] = float("inf")
+    out = torch.empty((5, n), device=dev())
+    tb.gguf(5, n, k, name).launch(x, wd, out)
+    want = x.double() @ tb.dequantize(wd, name, n, k).double().t()
+    assert torch.all(out[0] == 0) and torch.isnan(out[2]).all() and not torch.isfinite(out[3]).any()
+    for row in (1, 4):
+        assert float((out[row].double() - want[row]).norm() / want[row].norm()) < 1e-5
