@@ -1277,7 +1277,8 @@ GemvPlan plan_gemv_fast(int fmt, int xt, long long m, long long n, long long k,
   for (int per_sm = 2; per_sm >= 1; --per_sm) {
     if (force_per_sm && per_sm != force_per_sm) continue;
     const int slots = dev.sm_count * per_sm;
-    const int smem_limit = per_sm == 1 ? dev.max_smem_optin : (dev.max_smem_optin + 1024) / 2 - 1024;
+    // (one CTA per SM: the kernel's few static words count towards the same limit)
+    const int smem_limit = per_sm == 1 ? dev.max_smem_optin - 128 : (dev.max_smem_optin + 1024) / 2 - 1024;
     for (int splits = 1; splits <= nsb && splits <= 64; ++splits) {
       if (force_splits && splits != force_splits) continue;
       const int per = (nsb + splits - 1) / splits;

@@ -115,3 +115,10 @@ def test_scratch_regions_of_a_split_plan_are_aligned(m, n, k):
     """The converted activations lie behind splits x m x n partial sums and move in 16-byte units."""
     plan = tb.gemv_plan("q4_k", m, n, k)
     assert plan["k_splits"] > 1 and plan["scratch_bytes"] % 256 == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(2, 2048, 8192), (2, 12288, 8192), (8, 2048, 6144)])
+def test_plans_leave_room_for_static_shared_memory(m, n, k):
+    """The kernel has a few words of static shared memory besides what a plan asks for."""
+    plan = tb.gemv_plan("q4_k", m, n, k)
+    assert plan["pipelined"] and plan["smem_bytes"] + 128 <= 232448
