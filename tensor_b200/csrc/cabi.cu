@@ -276,6 +276,8 @@ int32_t tb200_gguf_device_status(uint32_t* status, TensorErrorV1* error) {
   if ((e = read_gemv_tc_status(&t, true)) != cudaSuccess) return cuda_fail(error, "reading GEMV status", e);
   if ((e = read_gemv_status(&a, true)) != cudaSuccess) return cuda_fail(error, "reading GEMV status", e);
   if (!a) a = t;
+  if ((e = read_gemv_frag_status(&t, true)) != cudaSuccess) return cuda_fail(error, "reading GEMV status", e);
+  if (!a) a = t;
   if ((e = read_gemm_status(&b, true)) != cudaSuccess) return cuda_fail(error, "reading GEMM status", e);
   if ((e = read_gemm_pair_status(&t, true)) != cudaSuccess) return cuda_fail(error, "reading GEMM status", e);
   if (!b) b = t;
@@ -305,15 +307,28 @@ int32_t tb200_gguf_dequant(int32_t format, const void* w, float* out, int64_t n,
 namespace {
 // Whether the default entry points run a decode GEMV on the kernel that keeps the activations in registers.
 bool use_frag(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k, int32_t variant, int out_count,
-              const PeerSync* peers, const Schedule* sched) {
+              const PeerSync* peers, const Schedule* sched, int prep_mode = kPrepNormal) {
   if (variant != TB200_VARIANT_AUTO || out_count != 1 || (peers && peers->flags) || sched) return false;
   if (!gemv_frag_supported(format, x_dtype, m, n, k)) return false;
-  // Where another kernel is ahead (us on B200, this one | that one): batch 1 on the integer dot-product units (Q6_K
-  // 4096 x 12288 19.8 | 13.7, Q8_0 12288 x 4096 19.4 | 12.4, Q4_0 13.8 | 9.7) and Q4_K's own pipeline with 2-byte
-  // activations (18944 x 3584: batch 1 17.7 | 10.9, batch 16 23.8 | 19.7).  Ahead here: Q6_K 4096 x 12288 at batch 16
-  // 27.6 | 46.5 (tensor memory), Q8_0 and Q4_0 12288 x 4096 at batch 8 19.8 | 132 and 14.7 | 102 (SIMT).
+  // Where another kernel is ahead (us on B200, this one | that one).  Batch 1: the integer dot-product units (Q6_K 4096 x
+  // 12288 18.8 | 13.7, Q8_0 12288 x 4096 18.7 | 12.4, Q4_0 13.6 | 9.7) and Q4_K's own pipeline (18944 x 3584 16.8 | 10.9).
+  // Against that: Q6_K 4096 x 12288 at batch 16 27.5 | 46.5 (tensor memory), Q8_0 and Q4_0 12288 x 4096 at batch 8
+  // 19.1 | 132 and 14.7 | 102 (SIMT), and all that neither of them takes.
   if (gemv_dp4a_supported(format, x_dtype, m, n, k)) return false;
-  if (format == kQ4_K && x_dtype != kF32) return false;
+  if (x_dtype == kF32 && format != kQ4_K && k <= 4096 && row_bytes(format, k) % 16 == 0) {
+    // The SIMT kernel that stages whole rows starts sooner than three fp16 parts are made (1024 x 4096, batch 1, Q6_K,
+    // Q8_0, Q4_0: 9.1 | 6.3, 8.8 | 5.5, 8.6 | 4.8; 12288 x 4096: 20.7 | 37.7, 22.5 | 26.3, 17.6 | 20.0).
+    if (n <= (m == 1 ? 4096 : m == 2 ? 1536 : 0)) return false;
+  }
+  if (format == kQ4_K && x_dtype != kF32) {
+    // (a list converts the activations of all its launches ahead, which leaves its own pipeline ahead: three
+    // projections of 18944 x 3584 at batches 1, 4 and 16 take 138 us so and 154 with the batch-16 launches here)
+    if (prep_mode != kPrepNormal) return false;
+    // Q4_K's pipeline fits two CTAs on an SM up to K = 3584 (12288 rows, batch 8 / 16: 13.5 | 11.4, 18.1 | 15.5) and one
+    // beyond (K = 4096 14.2 | 15.9, 19.3 | 24.7; K = 6144 19.0 | 20.4, 25.5 | 33.2); just above K = 4096 this kernel's
+    // clusters have only nine to eleven of sixteen warps busy (K = 5120 18.1 | 15.3, 24.6 | 30.4).
+    if (k <= 3584 || (m <= 8 && k > 4096 && k <= 5632)) return false;
+  }
   return !lookup_schedule(kOpGemv, format, m, n, k);  // a schedule recorded for the shape names the kernel it was searched on
 }
 
@@ -332,7 +347,7 @@ int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* 
   if (int32_t s = require_device(error, &dev)) return s;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const uint8_t* wp = static_cast<const uint8_t*>(w);
-  if (use_frag(format, x_dtype, m, n, k, variant, out.count, peers, sched)) {
+  if (use_frag(format, x_dtype, m, n, k, variant, out.count, peers, sched, prep_mode)) {
     if (prep_mode == kPrepOnly) return ok(error);  // (it converts the activations itself)
     cudaError_t e = launch_gemv_frag(format, x_dtype, x, wp, out, m, n, k, st);
     if (e == cudaSuccess) return ok(error);
@@ -661,7 +676,7 @@ static int32_t gemv_pair_sharded_impl(int32_t format, int32_t x_dtype, const voi
       }
     }
     if (n1 % kGemvTileRows == 0 &&
-        use_frag(format, x_dtype, m, n, k, variant, out_count, peers.flags ? &peers : nullptr, nullptr)) {
+        use_frag(format, x_dtype, m, n, k, variant, out_count, peers.flags ? &peers : nullptr, nullptr, prep_mode)) {
       if (prep_mode == kPrepOnly) return ok(error);
       OutSpec both = single_output(outs1[0] + col_offset1, out_ld);
       both.ptr2[0] = outs2[0] + col_offset2;

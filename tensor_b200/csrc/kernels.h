@@ -222,6 +222,7 @@ bool make_tensor_map_2d(void* map_out, TmaType type, const void* base, unsigned 
 bool allocation_range(const void* ptr, void** base, size_t* size);
 
 cudaError_t read_gemv_status(unsigned int* value, bool clear);
+cudaError_t read_gemv_frag_status(unsigned int* value, bool clear);
 cudaError_t read_gemv_tc_status(unsigned int* value, bool clear);
 cudaError_t read_gemm_status(unsigned int* value, bool clear);
 cudaError_t read_gemm_pair_status(unsigned int* value, bool clear);
