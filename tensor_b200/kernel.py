@@ -14,6 +14,7 @@ from __future__ import annotations
 import torch
 
 from . import ops
+from ._native import lib
 from .formats import get_format
 
 ARGUMENTS = ("x", "w", "out")
@@ -44,6 +45,8 @@ class GgufKernel:
         self.op = op
         self.variant = variant
         self.device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
+        self._type_id, self._x_id = self.format.type_id, ops._X_DTYPE_IDS[self.x_dtype]
+        self._x_count, self._out_count, self._w_count = self.m * self.k, self.m * self.n, self.weight_bytes
         self._scratch = None
         if op == "gemv" and torch.cuda.is_available():
             with torch.cuda.device(self.device):
@@ -76,6 +79,16 @@ class GgufKernel:
         return 2 * self.m * self.n * self.k
 
     # -- binding checks (executable.py:93-148) -----------------------------------------------------
+    def _ready(self, x, w, out) -> bool:
+        """Whether every check of :meth:`_check` passes, at the least cost; the details are left to it."""
+        device = self.device
+        return (isinstance(x, torch.Tensor) and isinstance(w, torch.Tensor) and isinstance(out, torch.Tensor)
+                and x.dtype == self.x_dtype and w.dtype == torch.uint8 and out.dtype == torch.float32
+                and x.numel() == self._x_count and w.numel() == self._w_count and out.numel() == self._out_count
+                and x.is_cuda and x.device == device and w.device == device and out.device == device
+                and x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
+                and not (x.data_ptr() | w.data_ptr() | out.data_ptr()) % ALIGNMENT)
+
     def _check(self, buffers):
         if len(buffers) != len(ARGUMENTS):
             raise ValueError(f"expected {len(ARGUMENTS)} arguments {ARGUMENTS}, got {len(buffers)}")
@@ -99,12 +112,18 @@ class GgufKernel:
 
     def launch(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, stream=None) -> torch.Tensor:
         """Enqueue on ``stream`` (default: torch's current stream of the device); asynchronous."""
-        self._check((x, w, out))
+        if not self._ready(x, w, out):
+            self._check((x, w, out))
+        device = x.device
+        handle = ops._stream_handle(device, stream)
         if self.op == "gemv":
-            ops.gemv(x, w, self.format, self.n, self.k, out=out, scratch=self._scratch,
-                     variant=self.variant, stream=stream)
+            scratch = self._scratch
+            ops._invoke(lib().tb200_gguf_gemv, device, self._type_id, self._x_id, x.data_ptr(), w.data_ptr(), out.data_ptr(),
+                        self.m, self.n, self.k, scratch.data_ptr() if scratch is not None else None,
+                        scratch.numel() if scratch is not None else 0, ops._VARIANTS[self.variant], handle)
         else:
-            ops.gemm(x, w, self.format, self.n, self.k, out=out, variant=self.variant, stream=stream)
+            ops._invoke(lib().tb200_gguf_gemm, device, self._type_id, self._x_id, x.data_ptr(), w.data_ptr(), out.data_ptr(),
+                        self.m, self.n, self.k, ops._VARIANTS[self.variant], handle)
         return out
 
     def __call__(self, x: torch.Tensor, w: torch.Tensor, stream=None) -> torch.Tensor:

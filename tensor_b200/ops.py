@@ -1,10 +1,12 @@
 """Host-side operators over torch CUDA tensors.  PyTorch supplies device memory and streams; the
-arithmetic is entirely in the C library (``tensor_b200/csrc``), reached through the reference's
-descriptor calling convention (``*_v1`` entry points of include/tensor_b200_gguf.h)."""
+arithmetic is entirely in the C library (``tensor_b200/csrc``), reached through its plain entry points
+(include/tensor_b200_gguf.h): filling in the reference's argument descriptors from Python took longer than
+a decode kernel runs."""
 
 from __future__ import annotations
 
 import ctypes
+from operator import index
 
 import torch
 
@@ -12,10 +14,13 @@ from . import abi
 from ._native import lib, raise_for_status
 from .formats import get_format
 
-_TORCH_DTYPE_IDS = {torch.uint8: 3, torch.float16: 10, torch.float32: 11, torch.bfloat16: 13}
+_X_DTYPE_IDS = {torch.float16: 10, torch.float32: 11, torch.bfloat16: 13}
 _VARIANTS = {"auto": 0, "simple": 1, "fast": 2, "mma": 3, "tc": 4, "dp4a": 5, 0: 0, 1: 1, 2: 2, 3: 3, 4: 4, 5: 5}
 _X_DTYPE_NAMES = {"float16": 10, "float32": 11, "bfloat16": 13, torch.float16: 10, torch.float32: 11, torch.bfloat16: 13}
 GEMV_LIST_MAX = 12
+
+# the current stream's handle without a Stream object around it
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
 
 
 def _require_cuda(name: str, t: torch.Tensor) -> None:
@@ -27,18 +32,9 @@ def _require_cuda(name: str, t: torch.Tensor) -> None:
         raise ValueError(f"{name} must be contiguous")
 
 
-def _buffer(name: str, t: torch.Tensor, shape=None) -> abi.TensorArgumentV1:
-    try:
-        dtype = _TORCH_DTYPE_IDS[t.dtype]
-    except KeyError:
-        raise ValueError(f"{name} has unsupported dtype {t.dtype}") from None
-    return abi.buffer_argument(t.data_ptr(), t.numel() * t.element_size(), dtype, t.device.index,
-                               shape if shape is not None else tuple(t.shape))
-
-
 def _stream_handle(device: torch.device, stream) -> int:
     if stream is None:
-        return torch.cuda.current_stream(device).cuda_stream
+        return _raw_stream(device.index)
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -52,12 +48,16 @@ def _same_device(*tensors) -> torch.device:
     return device
 
 
-def _invoke(fn, arguments, device, stream) -> None:
-    call, keep = abi.make_call(arguments, device.index, _stream_handle(device, stream))
+def _invoke(fn, device, *arguments) -> None:
+    """``fn(*arguments, &error)`` with ``device`` current, as the plain entry points want it."""
     error = abi.TensorErrorV1()
-    status = fn(ctypes.byref(call), ctypes.byref(error))
-    del keep
-    raise_for_status(status, error)
+    if torch.cuda.current_device() == device.index:
+        status = fn(*arguments, ctypes.byref(error))
+    else:
+        with torch.cuda.device(device):
+            status = fn(*arguments, ctypes.byref(error))
+    if status:
+        raise_for_status(status, error)
 
 
 def weight_bytes(encoding, n: int, k: int) -> int:
@@ -112,13 +112,15 @@ def dequantize(w: torch.Tensor, encoding, n: int, k: int, out: torch.Tensor | No
         out = torch.empty((n, k), dtype=torch.float32, device=w.device)
     _require_cuda("out", out)
     device = _same_device(w, out)
-    args = [_buffer("w", w, (w.numel(),)), _buffer("out", out, (n, k)),
-            abi.scalar_argument(n), abi.scalar_argument(k), abi.scalar_argument(fmt.type_id)]
-    _invoke(lib().tb200_gguf_dequant_v1, args, device, stream)
+    if out.dtype != torch.float32 or out.numel() != n * k:
+        raise ValueError(f"out must be float32 with {n * k} elements")
+    _invoke(lib().tb200_gguf_dequant, device, fmt.type_id, w.data_ptr(), out.data_ptr(), index(n), index(k),
+            _stream_handle(device, stream))
     return out
 
 
-def _matmul_args(x, w, out, fmt, m, n, k):
+def _check_matmul(x, w, out, fmt, m, n, k) -> int:
+    """Shapes and dtypes of a call; returns the id of the activation dtype."""
     _require_cuda("x", x)
     _require_cuda("w", w)
     _require_cuda("out", out)
@@ -130,7 +132,10 @@ def _matmul_args(x, w, out, fmt, m, n, k):
         raise ValueError(f"w holds {w.numel()} bytes; [{n}, {k}] in {fmt.name} needs {fmt.weight_bytes(n, k)}")
     if out.dtype != torch.float32 or out.numel() != m * n:
         raise ValueError(f"out must be float32 with {m * n} elements")
-    return [_buffer("x", x, (m, k)), _buffer("w", w, (w.numel(),)), _buffer("out", out, (m, n))]
+    try:
+        return _X_DTYPE_IDS[x.dtype]
+    except KeyError:
+        raise ValueError(f"unsupported activation dtype {x.dtype}") from None
 
 
 def _infer_m(x: torch.Tensor, k: int) -> int:
@@ -150,16 +155,16 @@ def gemv(x: torch.Tensor, w: torch.Tensor, encoding, n: int, k: int, out: torch.
     m = _infer_m(x, k)
     if out is None:
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-    args = _matmul_args(x, w, out, fmt, m, n, k)
+    x_dtype = _check_matmul(x, w, out, fmt, m, n, k)
     device = _same_device(x, w, out, scratch)
+    scratch_ptr, scratch_bytes = None, 0
     if scratch is not None:
         _require_cuda("scratch", scratch)
         if scratch.dtype != torch.uint8:
             raise ValueError("scratch must be uint8")
-        args.append(_buffer("scratch", scratch, (scratch.numel(),)))
-    args += [abi.scalar_argument(m), abi.scalar_argument(n), abi.scalar_argument(k),
-             abi.scalar_argument(fmt.type_id), abi.scalar_argument(_VARIANTS[variant])]
-    _invoke(lib().tb200_gguf_gemv_v1, args, device, stream)
+        scratch_ptr, scratch_bytes = scratch.data_ptr(), scratch.numel()
+    _invoke(lib().tb200_gguf_gemv, device, fmt.type_id, x_dtype, x.data_ptr(), w.data_ptr(), out.data_ptr(), m, index(n),
+            index(k), scratch_ptr, scratch_bytes, _VARIANTS[variant], _stream_handle(device, stream))
     return out
 
 
@@ -172,15 +177,11 @@ def gemm(x: torch.Tensor, w: torch.Tensor, encoding, n: int, k: int, out: torch.
         raise ValueError(f"the GEMM takes bfloat16 activations, got {x.dtype}")
     if out is None:
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-    args = _matmul_args(x, w, out, fmt, m, n, k)
+    x_dtype = _check_matmul(x, w, out, fmt, m, n, k)
     device = _same_device(x, w, out)
-    args += [abi.scalar_argument(m), abi.scalar_argument(n), abi.scalar_argument(k),
-             abi.scalar_argument(fmt.type_id), abi.scalar_argument(_VARIANTS[variant])]
-    _invoke(lib().tb200_gguf_gemm_v1, args, device, stream)
+    _invoke(lib().tb200_gguf_gemm, device, fmt.type_id, x_dtype, x.data_ptr(), w.data_ptr(), out.data_ptr(), m, index(n),
+            index(k), _VARIANTS[variant], _stream_handle(device, stream))
     return out
-
-
-_X_DTYPE_IDS = {torch.float16: 10, torch.float32: 11, torch.bfloat16: 13}
 
 
 PEER_WAIT, PEER_SIGNAL = 1, 2
@@ -212,14 +213,10 @@ def gemv_sharded(x: torch.Tensor, w: torch.Tensor, encoding, n: int, k: int, out
     table = (ctypes.c_void_p * max(len(ptrs), 1))(*ptrs)
     pads = [int(p) for p in (pad_ptrs or [])]
     pad_table = (ctypes.c_void_p * max(len(pads), 1))(*pads)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_gguf_gemv_sharded_sync(
-            fmt.type_id, x_dtype, x.data_ptr(), w.data_ptr(), table, len(ptrs), out_ld, col_offset, m, n, k,
-            scratch.data_ptr() if scratch is not None else None, scratch.numel() if scratch is not None else 0,
-            _VARIANTS[variant], pad_table if pads else None, rank, max(len(pads), 1), sync,
-            _stream_handle(device, stream), ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_gguf_gemv_sharded_sync, device, fmt.type_id, x_dtype, x.data_ptr(), w.data_ptr(), table,
+            len(ptrs), out_ld, col_offset, m, n, k, scratch.data_ptr() if scratch is not None else None,
+            scratch.numel() if scratch is not None else 0, _VARIANTS[variant], pad_table if pads else None, rank,
+            max(len(pads), 1), sync, _stream_handle(device, stream))
 
 
 def peer_sync(pad_ptrs, rank: int, device: torch.device, mode: int = PEER_WAIT | PEER_SIGNAL, stream=None) -> None:
@@ -227,11 +224,7 @@ def peer_sync(pad_ptrs, rank: int, device: torch.device, mode: int = PEER_WAIT |
     ``pad_ptrs[i]`` is the address of rank i's signal pad as mapped in this process."""
     ptrs = [int(p) for p in pad_ptrs]
     table = (ctypes.c_void_p * max(len(ptrs), 1))(*ptrs)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_peer_sync(table, rank, len(ptrs), mode, _stream_handle(device, stream),
-                                       ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_peer_sync, device, table, rank, len(ptrs), mode, _stream_handle(device, stream))
 
 
 def peer_barrier(pad_ptrs, rank: int, device: torch.device, stream=None) -> None:
@@ -310,13 +303,9 @@ class GemvList:
         self._keep[index] = (old_x if x is None else x, old_w if w is None else w, out)
 
     def launch(self, stream=None) -> None:
-        error = abi.TensorErrorV1()
-        with torch.cuda.device(self.device):
-            status = lib().tb200_gguf_gemv_list(
-                self._items, len(self._items), self.scratch.data_ptr(), self.scratch.numel(), self.variant,
-                self._pad_table if self._pads else None, self.rank, max(len(self._pads), 1), self.sync,
-                _stream_handle(self.device, stream), ctypes.byref(error))
-        raise_for_status(status, error)
+        _invoke(lib().tb200_gguf_gemv_list, self.device, self._items, len(self._items), self.scratch.data_ptr(),
+                self.scratch.numel(), self.variant, self._pad_table if self._pads else None, self.rank,
+                max(len(self._pads), 1), self.sync, _stream_handle(self.device, stream))
 
     __call__ = launch
 
@@ -335,11 +324,8 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6, out: torch
     if out.dtype != torch.bfloat16 or out.numel() != m * k:
         raise ValueError("out must be bfloat16 [m, k]")
     device = _same_device(x, weight, out)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_rmsnorm_bf16(x.data_ptr(), weight.data_ptr(), out.data_ptr(), m, k, float(eps),
-                                          _stream_handle(device, stream), ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_rmsnorm_bf16, device, x.data_ptr(), weight.data_ptr(), out.data_ptr(), m, k, float(eps),
+            _stream_handle(device, stream))
     return out
 
 
@@ -356,11 +342,8 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor | None = None, stream=None):
     if out.dtype != torch.bfloat16 or out.numel() != m * width:
         raise ValueError("out must be bfloat16 [m, width]")
     device = _same_device(gate_up, out)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_swiglu_bf16(gate_up.data_ptr(), out.data_ptr(), m, width, _stream_handle(device, stream),
-                                         ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_swiglu_bf16, device, gate_up.data_ptr(), out.data_ptr(), m, width, _stream_handle(device,
+            stream))
     return out
 
 
@@ -371,11 +354,8 @@ def residual_add(stream_buffer: torch.Tensor, delta: torch.Tensor, stream=None):
     if stream_buffer.dtype != torch.float32 or delta.dtype != torch.float32 or stream_buffer.numel() != delta.numel():
         raise ValueError("residual_add takes two float32 tensors of the same size")
     device = _same_device(stream_buffer, delta)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_residual_add(stream_buffer.data_ptr(), delta.data_ptr(), stream_buffer.numel(),
-                                          _stream_handle(device, stream), ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_residual_add, device, stream_buffer.data_ptr(), delta.data_ptr(), stream_buffer.numel(),
+            _stream_handle(device, stream))
     return stream_buffer
 
 
@@ -408,13 +388,9 @@ def gemv_pair(x: torch.Tensor, w1: torch.Tensor, n1: int, w2: torch.Tensor, n2: 
     if out.dtype != torch.float32 or out.numel() != m * (n1 + n2):
         raise ValueError(f"out must be float32 with {m * (n1 + n2)} elements")
     device = _same_device(x, w1, w2, out, scratch)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_gguf_gemv_pair(
-            fmt.type_id, x_dtype, x.data_ptr(), w1.data_ptr(), n1, w2.data_ptr(), n2, out.data_ptr(), m, k,
-            scratch.data_ptr() if scratch is not None else None, scratch.numel() if scratch is not None else 0,
-            _VARIANTS[variant], _stream_handle(device, stream), ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_gguf_gemv_pair, device, fmt.type_id, x_dtype, x.data_ptr(), w1.data_ptr(), n1,
+            w2.data_ptr(), n2, out.data_ptr(), m, k, scratch.data_ptr() if scratch is not None else None,
+            scratch.numel() if scratch is not None else 0, _VARIANTS[variant], _stream_handle(device, stream))
     return out
 
 
@@ -445,11 +421,7 @@ def gemv_pair_sharded(x: torch.Tensor, w1: torch.Tensor, n1: int, w2: torch.Tens
     table2 = (ctypes.c_void_p * max(count, 1))(*[int(p) for p in out2_ptrs])
     pads = [int(p) for p in (pad_ptrs or [])]
     pad_table = (ctypes.c_void_p * max(len(pads), 1))(*pads)
-    error = abi.TensorErrorV1()
-    with torch.cuda.device(device):
-        status = lib().tb200_gguf_gemv_pair_sharded_sync(
-            fmt.type_id, x_dtype, x.data_ptr(), w1.data_ptr(), n1, w2.data_ptr(), n2, table1, table2, count, out_ld,
-            col_offset1, col_offset2, m, k, scratch.data_ptr() if scratch is not None else None,
-            scratch.numel() if scratch is not None else 0, _VARIANTS[variant], pad_table if pads else None, rank,
-            max(len(pads), 1), sync, _stream_handle(device, stream), ctypes.byref(error))
-    raise_for_status(status, error)
+    _invoke(lib().tb200_gguf_gemv_pair_sharded_sync, device, fmt.type_id, x_dtype, x.data_ptr(), w1.data_ptr(), n1,
+            w2.data_ptr(), n2, table1, table2, count, out_ld, col_offset1, col_offset2, m, k, scratch.data_ptr() if
+            scratch is not None else None, scratch.numel() if scratch is not None else 0, _VARIANTS[variant],
+            pad_table if pads else None, rank, max(len(pads), 1), sync, _stream_handle(device, stream))
