@@ -955,10 +955,10 @@ ListUnits list_units(const TB200GemvItem* items, int count, const TcLaunchItem* 
       const bool pipelined = both.supported && both.k_splits == 1 && items[i].n % kGemvTileRows == 0;
       pair = pipelined || (items[i].n % kGemvTileRows == 0 &&
                            use_frag(items[i].format, items[i].x_dtype, items[i].m, items[i].n + items[i + 1].n, items[i].k,
-                                    variant, items[i].out_count, nullptr, nullptr));
+                                    variant, items[i].out_count, nullptr, nullptr, kPrepDone));
       if (pipelined) need = both.scratch_bytes;
       else if (pair)
-        need = std::max<long long>(need, tb200_gguf_gemv_scratch_bytes(items[i].format, items[i + 1].m, items[i + 1].n, items[i + 1].k));
+        need = (need + 255) / 256 * 256 + tb200_gguf_gemv_scratch_bytes(items[i].format, items[i + 1].m, items[i + 1].n, items[i + 1].k);
     }
     need = (need + 255) / 256 * 256;
     u.first[u.count] = i;

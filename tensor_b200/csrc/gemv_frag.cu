@@ -259,15 +259,24 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
         f.b[s][t][1] = __byte_perm(lo, hi, 0x7632);
       }
       if constexpr (XT == kBF16) {
-        uint32_t mx = 0;
+        uint32_t both = 0;
 #pragma unroll
         for (int s = 0; s < 16; ++s)
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const uint32_t lo = f.b[s][t][j] & 0x7FFFu, hi = (f.b[s][t][j] >> 16) & 0x7FFFu;
-            if (lo < 0x7F80u) mx = max(mx, lo);
-            if (hi < 0x7F80u) mx = max(mx, hi);
-          }
+          for (int j = 0; j < 2; ++j)
+            asm("max.u16x2 %0, %0, %1;" : "+r"(both) : "r"(f.b[s][t][j] & 0x7FFF7FFFu));
+        uint32_t mx = max(both & 0xFFFFu, both >> 16);
+        if (__any_sync(0xffffffffu, mx >= 0x7F80u)) {  // the scale follows the finite values
+          mx = 0;
+#pragma unroll
+          for (int s = 0; s < 16; ++s)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const uint32_t lo = f.b[s][t][j] & 0x7FFFu, hi = (f.b[s][t][j] >> 16) & 0x7FFFu;
+              if (lo < 0x7F80u) mx = max(mx, lo);
+              if (hi < 0x7F80u) mx = max(mx, hi);
+            }
+        }
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         if (mx >> 7) scale = scale_for(mx >> 7);
@@ -283,17 +292,18 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
     f.u[t][0] = __shfl_sync(0xffffffffu, unscale, 8 * tig);
     f.u[t][1] = __shfl_sync(0xffffffffu, unscale, 8 * tig + 4);
     if constexpr (FMT == kQ4_K) {
+      // group sums by MMA: row i of A is one where lane i of a column feeds it, so that row i of D is the sum over lane
+      // i's elements; lane (column, i) then fetches its own from the lane that holds it (an infinity or a NaN reaches
+      // every group of its column, whose result is NaN anyway)
+      const uint32_t ones = gid == tig ? 0x3C003C00u : 0u;
       float hi[2], lo[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        float sum = 0.f;
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const float2 p = __half22float2(*reinterpret_cast<const __half2*>(&f.b[8 * h + s][t][0]));
-          const float2 q = __half22float2(*reinterpret_cast<const __half2*>(&f.b[8 * h + s][t][1]));
-          sum += (p.x + q.x) + (p.y + q.y);
-        }
-        sum *= 0.015625f;
+        for (int s = 0; s < 8; ++s) ptx::mma16816<true>(c, ones, 0u, ones, 0u, f.b[8 * h + s][t][0], f.b[8 * h + s][t][1], c);
+        const float even = __shfl_sync(0xffffffffu, c[0], 4 * tig + (gid >> 1)), odd = __shfl_sync(0xffffffffu, c[1], 4 * tig + (gid >> 1));
+        const float sum = (gid & 1 ? odd : even) * 0.015625f;
         hi[h] = __half2float(__float2half_rn(sum));
         lo[h] = sum - hi[h];
       }
@@ -626,7 +636,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_frag_kernel(const FragArgs a
   // what the owner does: the partial tiles of tile `which` (buffer b, for the use-th time) added in K order
   auto add_up = [&](int which, int b, int use, int to_slot, int share) {
     if (ok && !ptx::mbar_wait(&full[b], use & 1)) {
-      report_timeout(0x90000u);
+      report_timeout(0xA0000u);
       ok = false;
     }
     if (!ok) return;
@@ -662,7 +672,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_frag_kernel(const FragArgs a
       float acc[NT][4];
       tile_item<FMT, NT>(f, stage, ln, tig, acc);
       if (use > 0 && ok && !ptx::mbar_wait(&empty[buf], (use - 1) & 1)) {
-        report_timeout(0xA0000u);
+        report_timeout(0xB0000u);
         ok = false;
       }
       const uint32_t to = mine + (uint32_t)buf * red_bytes;
