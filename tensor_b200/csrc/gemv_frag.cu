@@ -21,6 +21,11 @@
 //
 // The warps of a CTA cover up to 4096 of K; a longer K is spread over the CTAs of a cluster, which add their sums through
 // distributed shared memory.  All sums are added in K order: no scratch, no atomics, the same bits on every launch.
+//
+// What bounds it is instruction issue: about 500 warp instructions per 16 x 256 weights (Q4_K, batch 8), half of the issue
+// slots used, DRAM at a fifth of its rate.  Measured (us, this kernel | the one before; graph replay over weights larger
+// than the L2): Q6_K 4096 x 12288 at batch 4 / 16 19.1 | 39.7 and 26.2 | 46.5 (tensor memory), Q8_0 12288 x 4096 18.5 | 72.3
+// and 23.6 | 228, Q4_0 13.6 | 60.9 and 18.5 | 178 (SIMT), Q4_K 24576 x 4096 20.9 | 24.5 and 28.3 | 41.2 (gemv_mma.cu).
 #include <cuda_fp16.h>
 
 #include <algorithm>
