@@ -324,10 +324,14 @@ bool use_frag(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k, 
     // (a list converts the activations of all its launches ahead, which leaves its own pipeline ahead: three
     // projections of 18944 x 3584 at batches 1, 4 and 16 take 138 us so and 154 with the batch-16 launches here)
     if (prep_mode != kPrepNormal) return false;
-    // Q4_K's pipeline fits two CTAs on an SM up to K = 3584 (12288 rows, batch 8 / 16: 13.5 | 11.4, 18.1 | 15.5) and one
-    // beyond (K = 4096 14.2 | 15.9, 19.3 | 24.7; K = 6144 19.0 | 20.4, 25.5 | 33.2); just above K = 4096 this kernel's
-    // clusters have only nine to eleven of sixteen warps busy (K = 5120 18.1 | 15.3, 24.6 | 30.4).
-    if (k <= 3584 || (m <= 8 && k > 4096 && k <= 5632)) return false;
+    // Q4_K's own pipeline fits two CTAs on an SM up to K = 3584, where it is ahead (12288 x 3584, batch 8 / 16: 13.5 |
+    // 11.4, 18.1 | 15.5), and one beyond.  Two column tiles (m > 8): 7296 rows, batch 16, K = 3840 13.0 | 21.1, 8192 21.2 |
+    // 26.7, 14336 35.3 | 45.4, 28160 70 | 74; not so for few rows at batches just above 8 (2048 x 4096, batch 12: 8.1 |
+    // 7.3).  One column tile: only where K fills all sixteen warps of every CTA (7296 rows, batch 8, K = 4096 9.9 | 12.1,
+    // 8192 16.3 | 21.5, 12288 22.2 | 23.0, but 7168 15.4 | 15.1, 14336 26.7 | 23.5, 18944 with fifteen and clusters of five
+    // 32.9 | 33.3, 28160 51 | 47), and with rows enough to pay for a cluster (2048 x 8192, batch 2: 8.2 | 7.4).
+    if (k <= 3584) return false;
+    if (m > 8 ? m <= 12 && n <= 2048 && k <= 4096 : k % 4096 || k > 12288 || (k > 4096 && n < 4096)) return false;
   }
   return !lookup_schedule(kOpGemv, format, m, n, k);  // a schedule recorded for the shape names the kernel it was searched on
 }

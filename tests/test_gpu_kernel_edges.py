@@ -98,7 +98,7 @@ def test_split_gemv_with_odd_row_counts(m, n, k):
 @pytest.mark.parametrize("m,n,blocks,x", [
     (2, 1, 1, "bf16"), (3, 15, 2, "f16"), (8, 17, 9, "bf16"), (9, 100, 5, "bf16"), (16, 2500, 3, "f16"), (16, 33, 17, "bf16"),
     (5, 513, 33, "bf16"), (7, 20, 112, "bf16"), (1, 31, 16, "f32"), (2, 300, 7, "f32"), (3, 49, 40, "f32"), (16, 64, 11, "f32"),
-    (1, 130, 15, "bf16"),
+    (1, 130, 15, "bf16"), (8, 100, 16, "bf16"), (12, 2049, 16, "bf16"),
 ])
 def test_gemv_frag_edges(name, m, n, blocks, x):
     # blocks counts 256 weights for the K-quants and 32 for the others (times 5 where that leaves a part of a slice)
@@ -135,3 +135,20 @@ def test_gemv_frag_special_values(name):
     assert torch.all(out[0] == 0) and torch.isnan(out[2]).all() and not torch.isfinite(out[3]).any()
     for row in (1, 4):
         assert float((out[row].double() - want[row]).norm() / want[row].norm()) < 1e-5
+
+
+@pytest.mark.parametrize("name,k", [("q6_k", 768), ("q8_0", 4128), ("q4_0", 992), ("q4_k", 4096)])
+@pytest.mark.parametrize("n1,n2", [(48, 33), (16, 1), (40, 24)])
+def test_gemv_frag_two_weights(name, k, n1, n2):
+    """A grouped launch (first weight of whole tiles) and the two launches it stands for agree."""
+    m = 6
+    x = to_dev(oracle.make_activations(m, k, seed=1, dtype="bf16"), torch.bfloat16)
+    ws = [to_dev(oracle.make_weights(name, n, k, seed=n)) for n in (n1, n2)]
+    out = torch.full((m, n1 + n2), float("nan"), device=dev())
+    tb.ops.gemv_pair(x, ws[0], n1, ws[1], n2, name, k, out=out)
+    want = x.double() @ torch.cat([tb.dequantize(w, name, n, k) for w, n in zip(ws, (n1, n2))]).double().t()
+    assert float((out.double() - want).norm() / want.norm()) < 1e-5  # exact operands, fp32 sums: a few sqrt(K) 2^-24
+    parts = [torch.empty((m, n), device=dev()) for n in (n1, n2)]
+    for w, n, part in zip(ws, (n1, n2), parts):
+        tb.gemv(x, w, name, n, k, out=part)
+    assert float((out - torch.cat(parts, 1)).norm() / out.norm()) < 1e-5
