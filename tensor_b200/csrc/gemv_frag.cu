@@ -17,7 +17,8 @@
 //    sums (kept as two fp16 parts); the other formats' centred integers, with d (and Q6_K's 8-bit scale, whose product
 //    with the quant would not fit 11 bits) applied to the fp32 accumulators of a scale group;
 //  * bf16 activations are multiplied by one power of two per (row, slice) and then fit fp16 exactly (values down to
-//    2^-29 of the largest); fp32 ones are split exactly into three fp16 parts on three columns.
+//    2^-29 of the largest; fp16 ones, for Q4_K, by one that keeps them exact); fp32 ones are split exactly into three
+//    fp16 parts on three columns.
 //
 // The warps of a CTA cover up to 4096 of K; a longer K is spread over the CTAs of a cluster, which add their sums through
 // distributed shared memory.  All sums are added in K order: no scratch, no atomics, the same bits on every launch.
@@ -263,7 +264,11 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
         f.b[s][t][0] = __byte_perm(lo, hi, 0x5410);
         f.b[s][t][1] = __byte_perm(lo, hi, 0x7632);
       }
-      if constexpr (XT == kBF16) {
+      // fp16 values are MMA operands as they are; only Q4_K scales them, because its group sums become fp16 parts below:
+      // unscaled, the low part of a sum / 64 falls under fp16's smallest step from magnitudes of about 2^-6 on (error
+      // against fp64 at 4 x 2048 x 4096, weights of mean zero: 3e-5 at 2^-7, 2e-2 at 2^-16)
+      if constexpr (XT == kBF16 || FMT == kQ4_K) {
+        constexpr uint32_t kNonFinite = XT == kBF16 ? 0x7F80u : 0x7C00u;
         uint32_t both = 0;
 #pragma unroll
         for (int s = 0; s < 16; ++s)
@@ -271,26 +276,38 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
           for (int j = 0; j < 2; ++j)
             asm("max.u16x2 %0, %0, %1;" : "+r"(both) : "r"(f.b[s][t][j] & 0x7FFF7FFFu));
         uint32_t mx = max(both & 0xFFFFu, both >> 16);
-        if (__any_sync(0xffffffffu, mx >= 0x7F80u)) {  // the scale follows the finite values
+        if (__any_sync(0xffffffffu, mx >= kNonFinite)) {  // the scale follows the finite values
           mx = 0;
 #pragma unroll
           for (int s = 0; s < 16; ++s)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
               const uint32_t lo = f.b[s][t][j] & 0x7FFFu, hi = (f.b[s][t][j] >> 16) & 0x7FFFu;
-              if (lo < 0x7F80u) mx = max(mx, lo);
-              if (hi < 0x7F80u) mx = max(mx, hi);
+              if (lo < kNonFinite) mx = max(mx, lo);
+              if (hi < kNonFinite) mx = max(mx, hi);
             }
         }
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        if (mx >> 7) scale = scale_for(mx >> 7);
+        if constexpr (XT == kBF16) {
+          if (mx >> 7) scale = scale_for(mx >> 7);
 #pragma unroll
-        for (int s = 0; s < 16; ++s)
+          for (int s = 0; s < 16; ++s)
 #pragma unroll
-          for (int j = 0; j < 2; ++j)
-            f.b[s][t][j] = pack_f16(__uint_as_float(f.b[s][t][j] << 16) * scale,
-                                    __uint_as_float(f.b[s][t][j] & 0xFFFF0000u) * scale);
+            for (int j = 0; j < 2; ++j)
+              f.b[s][t][j] = pack_f16(__uint_as_float(f.b[s][t][j] << 16) * scale,
+                                      __uint_as_float(f.b[s][t][j] & 0xFFFF0000u) * scale);
+        } else {
+          // upwards only and by at most 2^15, so that the product is exact; a sum / 64 of values that the cap leaves
+          // small is still a multiple of 2^-15
+          const int sh = min(15, max(0, 29 - (int)(mx >> 10)));
+          scale = __uint_as_float((uint32_t)(127 + sh) << 23);
+          const uint32_t scale2 = (uint32_t)(15 + sh) * 0x04000400u;
+#pragma unroll
+          for (int s = 0; s < 16; ++s)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) f.b[s][t][j] = hmul2(f.b[s][t][j], scale2);
+        }
       }
     }
     const float unscale = __uint_as_float((254u << 23) - __float_as_uint(scale));  // both are powers of two

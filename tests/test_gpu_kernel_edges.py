@@ -119,6 +119,32 @@ def test_gemv_frag_edges(name, m, n, blocks, x):
     assert float((out.double() - want).norm() / want.norm()) < (2e-5 if name == "q4_k" else 1e-5)
 
 
+def balanced_q4_k(n, k, seed):
+    """Q4_K blocks as a quantised weight of mean zero has them: every group's minimum is 7.5 times its scale."""
+    raw = oracle.make_weights("q4_k", n, k, seed=seed).reshape(-1, 144)
+    d = np.ascontiguousarray(raw[:, 0:2]).view(np.float16).astype(np.float32)
+    raw[:, 2:4] = (7.5 * d).astype(np.float16).view(np.uint8)
+    raw[:, 8:12] = raw[:, 4:8]
+    raw[:, 12:16] = (raw[:, 12:16] & 15) * 17
+    return raw.reshape(-1)
+
+
+@pytest.mark.parametrize("exponent", [0, -4, -7, -10, -12, -14, -16])
+@pytest.mark.parametrize("m,k", [(4, 4096), (16, 4096), (4, 12288), (16, 12288)])
+def test_gemv_frag_q4k_small_f16_activations(m, k, exponent):
+    """The minimums' share of a result is as large as the quants': group sums keep their precision at every magnitude."""
+    n = 272
+    wd = to_dev(balanced_q4_k(n, k, seed=k))
+    gen = torch.Generator(device=dev()).manual_seed(m)
+    x = (torch.randn((m, k), device=dev(), generator=gen) * 2.0 ** exponent).to(torch.float16)
+    x[m - 1, 256:512] = 0
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gguf(m, n, k, "q4_k", x_dtype="float16").launch(x, wd, out)
+    want = x.double() @ tb.dequantize(wd, "q4_k", n, k).double().t()
+    # exact operands: fp32 sums of up to 12288 products, a few times sqrt(K) 2^-24 = 6.6e-6 of terms about twice the result
+    assert float((out.double() - want).norm() / want.norm()) < 2e-5
+
+
 @pytest.mark.parametrize("name", ["q8_0", "q4_0", "q6_k"])
 def test_gemv_frag_special_values(name):
     """Rows with an infinity or a NaN stay with themselves; zero and tiny rows keep their scale."""
