@@ -44,6 +44,7 @@ constexpr int kMaxRawStages = 6;
 constexpr int kMaxTokens = 256;
 constexpr int kThreads = 24 * 32;
 constexpr int kDecodeWarp0 = 8;
+constexpr int kGroups = 5;       // of four warps that wait together: four that decode, one that drains
 constexpr int kSmemLimit = 232448;
 constexpr int kBarrierBytes = 1024;
 constexpr int kRing = kSmemLimit - 1024 /*alignment*/ - kBarrierBytes;  // activation and raw stages
@@ -147,20 +148,34 @@ __device__ __forceinline__ bool wait_all(const uint32_t (&bar)[4], const uint32_
 }
 // The same for a group of four warps: one polls, the others wait at a hardware barrier.  (With every decode warp
 // polling, the polls queue up in front of the MMA warp's own and a satisfied wait takes 200 clocks there.)
-__device__ __forceinline__ bool wait_group(uint64_t* bar, uint32_t parity, int group, volatile int* gave_up) {
-  if ((threadIdx.x & 96) == 0 && !wait_bar(bar, parity)) *gave_up = 1;
-  ptx::bar_sync(1 + group, 128);
-  return *gave_up == 0;
-}
-__device__ __forceinline__ bool wait_group2(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1, int group, volatile int* gave_up) {
-  if ((threadIdx.x & 96) == 0) {
-    const uint32_t b0 = ptx::smem_addr(bar0), b1 = ptx::smem_addr(bar1);
-    const uint32_t bar[4] = {b0, b1, b0, b1}, par[4] = {parity0, parity1, parity0, parity1};
-    if (!wait_all(bar, par)) *gave_up = 1;
+// `late`: two words a group, in turn, that say whether a wait has run out.  Only the group's own poller writes them, before
+// the barrier, and not again before every warp of the group has passed the next one: the four read the same and go on or
+// leave together.  (A word shared with other groups could change between two of the reads, and part of a group would
+// wait for the rest at the next barrier without end.)
+struct GroupWait {
+  uint32_t late;  // shared address of the word of this wait; the other one is 4 bytes on or back
+  int group;
+  __device__ __forceinline__ void ran_out() { asm volatile("st.shared.u32 [%0], 1;" ::"r"(late) : "memory"); }
+  __device__ __forceinline__ bool verdict() {
+    ptx::bar_sync(1 + group, 128);
+    uint32_t word;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(word) : "r"(late) : "memory");
+    late ^= 4u;
+    return word == 0;
   }
-  ptx::bar_sync(1 + group, 128);
-  return *gave_up == 0;
-}
+  __device__ __forceinline__ bool one(uint64_t* bar, uint32_t parity) {
+    if ((threadIdx.x & 96) == 0 && !wait_bar(bar, parity)) ran_out();
+    return verdict();
+  }
+  __device__ __forceinline__ bool two(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1) {
+    if ((threadIdx.x & 96) == 0) {
+      const uint32_t b0 = ptx::smem_addr(bar0), b1 = ptx::smem_addr(bar1);
+      const uint32_t bar[4] = {b0, b1, b0, b1}, par[4] = {parity0, parity1, parity0, parity1};
+      if (!wait_all(bar, par)) ran_out();
+    }
+    return verdict();
+  }
+};
 // Activation half-tile into this CTA's shared memory, counted on the pair's first CTA's barrier (no multicast).
 __device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t leader_bar) {
   asm volatile(
@@ -443,8 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* acc_full = raw_empty + kMaxRawStages;  // [2] an accumulator set is complete (both CTAs)
   uint64_t* acc_empty = acc_full + 2;              // [2] both CTAs have drained it (first CTA)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_slot + 1);  // a wait of this CTA has run out
-  static_assert((2 * kMaxAStages + 2 * kMaxBStages + 2 * kMaxRawStages + 4) * 8 + 8 <= kBarrierBytes, "barriers");
+  uint32_t* late = tmem_slot + 2;  // [kGroups][2], see GroupWait
+  static_assert((2 * kMaxAStages + 2 * kMaxBStages + 2 * kMaxRawStages + 4) * 8 + 8 + 8 * kGroups <= kBarrierBytes, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();      // CTA of the cluster
@@ -476,7 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_init(&acc_full[b], 1);
       ptx::mbar_init(&acc_empty[b], 2 * 4);
     }
-    *gave_up = 0;
+    for (int i = 0; i < 2 * kGroups; ++i) late[i] = 0u;
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&map_x);
     if (a.tiled) ptx::prefetch_tensormap(&map_w);
@@ -639,6 +654,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int r = (warp & 3) * 32 + lane;                         // row of this CTA's half of the tile = TMEM lane
     const uint32_t full_leader = map_rank(ptx::smem_addr(full_a), leader);
     const uint32_t tmem_row = tmem_a + ((uint32_t)((warp & 3) * 32) << 16);
+    GroupWait group{ptx::smem_addr(late + 2 * j), j};
     int s = 0, base = 0;
     uint32_t parity = 0;
     bool ok = true;
@@ -652,8 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         // with two stages of its own a group asks for the raw bytes and the stage in one go (T = 128, Q6_K: 265 -> 249 us
         // at M = 2048, N = 12288, K = 4096); with one the stage is waited for after the decode
         const bool together = live && a.a_log == 3;
-        if (together ? !wait_group2(&raw_full[s], parity, &empty_a[sa], a_parity, j, gave_up)
-                     : !wait_group(&raw_full[s], parity, j, gave_up)) {
+        if (together ? !group.two(&raw_full[s], parity, &empty_a[sa], a_parity) : !group.one(&raw_full[s], parity)) {
           report_timeout(0x70000u | (unsigned)c);
           ok = false;
           break;
@@ -669,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) ptx::mbar_arrive(&raw_empty[s]);  // the row's bytes are in registers
         if (++s == a.raw_stages) s = 0, parity ^= 1;
         if (!live) continue;
-        if (!together && !wait_group(&empty_a[sa], a_parity, j, gave_up)) {
+        if (!together && !group.one(&empty_a[sa], a_parity)) {
           report_timeout(0x30000u | (unsigned)kb);
           ok = false;
           break;
@@ -686,10 +701,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---------------- epilogue: the accumulators of one tile while the next one's are being filled ----------------
     ptx::grid_dependency_wait();  // the kernel before may still read or write the output
     const int quarter = warp & 3;
+    GroupWait group{ptx::smem_addr(late + 2 * 4), 4};
     int t = 0;
     for (int tile = cluster; tile < a.tiles; tile += clusters, ++t) {
       const int b = a.acc_sets == 2 ? (t & 1) : 0, use = a.acc_sets == 2 ? (t >> 1) : t;
-      if (!wait_group(&acc_full[b], use & 1, 4, gave_up)) {
+      if (!group.one(&acc_full[b], use & 1)) {
         report_timeout(0x40000u);
         break;
       }
@@ -729,7 +745,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (warp >= 4 && warp < 8) {
       ptx::grid_dependency_wait();
       const int quarter = warp & 3;
-      if (!wait_group(&acc_full[0], 0, 4, gave_up)) {
+      if (!GroupWait{ptx::smem_addr(late + 2 * 4), 4}.one(&acc_full[0], 0)) {
         report_timeout(0x40000u);
       } else {
         ptx::tc_fence_after();

@@ -242,3 +242,20 @@ def test_gemv_pair_validates_before_touching_a_device():
     assert call(n2=-1) == 2
     assert call(variant=6) == 2
     assert call() == 3  # well-formed: stops at the missing device, never computes on the CPU
+
+
+def test_group_waits_of_the_paired_gemm_end_together():
+    """Four warps that meet at a hardware barrier after a wait go on or leave together.  A word that other groups write as
+    well could change between two of the four reads and leave part of a group at the next barrier without end: the word a
+    group reads after its barrier is its own, one of two in turn.  (A wait cannot be made to run out in that kernel
+    without a fault, so its source is looked at.)"""
+    source = open(os.path.join(ROOT, "tensor_b200", "csrc", "gemm_pair.cu")).read()
+    assert "gave_up" not in source
+    body = source[source.index("struct GroupWait {"):]
+    body = body[:body.index("\n};")]
+    assert body.count(" ran_out();") == 2 and body.count("return verdict();") == 2
+    verdict = body[body.index("bool verdict()"):body.index("bool one(")]
+    assert verdict.index("bar_sync(1 + group") < verdict.index("ld.shared.u32") < verdict.index("late ^= 4u")
+    kernel = source[source.index("__global__"):]
+    groups = re.findall(r"GroupWait(?: group)?\{ptx::smem_addr\(late \+ 2 \* (\w+)\), (\w+)\}", kernel)
+    assert len(groups) >= 3 and all(words == barrier for words, barrier in groups)
