@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* acc_empty = acc_full + 2;              // [2] both CTAs have drained it (first CTA)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   uint32_t* late = tmem_slot + 2;  // [kGroups][2], see GroupWait
+  volatile uint32_t* gave_up = tmem_slot + 1;  // some wait of this CTA has run out (read once all its warps are through)
   static_assert((2 * kMaxAStages + 2 * kMaxBStages + 2 * kMaxRawStages + 4) * 8 + 8 + 8 * kGroups <= kBarrierBytes, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -492,6 +493,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       ptx::mbar_init(&acc_empty[b], 2 * 4);
     }
     for (int i = 0; i < 2 * kGroups; ++i) late[i] = 0u;
+    *gave_up = 0u;
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&map_x);
     if (a.tiled) ptx::prefetch_tensormap(&map_w);
@@ -529,6 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (last >= a.b_stages) last -= a.b_stages;
           if (!wait_bar(&empty_b[last], last_parity)) {
             report_timeout(0x10000u | (unsigned)kb);
+            *gave_up = 1u;
             ok = false;
             break;
           }
@@ -555,6 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int b = a.acc_sets == 2 ? (t & 1) : 0, use = a.acc_sets == 2 ? (t >> 1) : t;
         if (!wait_bar(&acc_empty[b], (use & 1) ^ 1)) {
           report_timeout(0x50000u | (unsigned)t);
+          *gave_up = 1u;
           break;
         }
         ptx::tc_fence_after();
@@ -569,6 +573,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint32_t par[4] = {parity, (uint32_t)(seq >> a.a_log) & 1u, parity1, (uint32_t)(seq1 >> a.a_log) & 1u};
           if (!wait_all(bar, par)) {
             report_timeout(0x20000u | (unsigned)kb);
+            *gave_up = 1u;
             ok = false;
             break;
           }
@@ -607,6 +612,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (it == a.raw_stages) ptx::grid_dependency_wait();
         if (!wait_bar(&raw_empty[s], parity)) {
           report_timeout(0x60000u | (unsigned)c);
+          *gave_up = 1u;
           ok = false;
           break;
         }
@@ -670,6 +676,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const bool together = live && a.a_log == 3;
         if (together ? !group.two(&raw_full[s], parity, &empty_a[sa], a_parity) : !group.one(&raw_full[s], parity)) {
           report_timeout(0x70000u | (unsigned)c);
+          *gave_up = 1u;
           ok = false;
           break;
         }
@@ -686,6 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (!live) continue;
         if (!together && !group.one(&empty_a[sa], a_parity)) {
           report_timeout(0x30000u | (unsigned)kb);
+          *gave_up = 1u;
           ok = false;
           break;
         }
@@ -707,6 +715,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int b = a.acc_sets == 2 ? (t & 1) : 0, use = a.acc_sets == 2 ? (t >> 1) : t;
       if (!group.one(&acc_full[b], use & 1)) {
         report_timeout(0x40000u);
+        *gave_up = 1u;
         break;
       }
       ptx::tc_fence_after();
@@ -747,6 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const int quarter = warp & 3;
       if (!GroupWait{ptx::smem_addr(late + 2 * 4), 4}.one(&acc_full[0], 0)) {
         report_timeout(0x40000u);
+        *gave_up = 1u;
       } else {
         ptx::tc_fence_after();
         for (int col = 0; col < tok_end; col += 16) {
@@ -779,6 +789,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncwarp();
   ptx::tc_fence_before();
   __syncthreads();
+  if (*gave_up) {
+    // copies and MMAs still in flight get 50 us to end before the memory is given back, in both CTAs of the pair
+    const uint64_t start = ptx::global_timer_ns();
+    while (ptx::global_timer_ns() - start < 50000ull) __nanosleep(1000);
+    __syncwarp();
+  }
   cluster_sync();  // nobody may still arrive at, or read, a CTA that has left
   if (warp == 1) {
     ptx::tc_fence_after();

@@ -250,7 +250,6 @@ def test_group_waits_of_the_paired_gemm_end_together():
     group reads after its barrier is its own, one of two in turn.  (A wait cannot be made to run out in that kernel
     without a fault, so its source is looked at.)"""
     source = open(os.path.join(ROOT, "tensor_b200", "csrc", "gemm_pair.cu")).read()
-    assert "gave_up" not in source
     body = source[source.index("struct GroupWait {"):]
     body = body[:body.index("\n};")]
     assert body.count(" ran_out();") == 2 and body.count("return verdict();") == 2
@@ -259,3 +258,14 @@ def test_group_waits_of_the_paired_gemm_end_together():
     kernel = source[source.index("__global__"):]
     groups = re.findall(r"GroupWait(?: group)?\{ptx::smem_addr\(late \+ 2 \* (\w+)\), (\w+)\}", kernel)
     assert len(groups) >= 3 and all(words == barrier for words, barrier in groups)
+
+
+def test_the_paired_gemm_lets_copies_land_after_a_wait_that_ran_out():
+    """Whichever role gives up, the CTA holds its memory until copies and MMAs in flight have ended.  (Source only, as
+    above.)"""
+    source = open(os.path.join(ROOT, "tensor_b200", "csrc", "gemm_pair.cu")).read()
+    kernel = source[source.index("__global__"):source.index("// ---- host side")]
+    reports = re.findall(r"report_timeout\([^;]*;\s*(\S[^;]*;)", kernel)
+    assert len(reports) >= 8 and all(then == "*gave_up = 1u;" for then in reports)
+    end = kernel[kernel.rindex("__syncthreads();"):]
+    assert end.index("if (*gave_up)") < end.index("global_timer_ns") < end.index("cluster_sync();") < end.index("tcgen05.dealloc")
