@@ -126,6 +126,11 @@ int64_t tb200_gguf_gemv_scratch_bytes(int32_t format, int64_t m, int64_t n, int6
 int32_t tb200_gguf_gemv_plan(int32_t format, int64_t m, int64_t n, int64_t k, int64_t scratch_bytes,
                              int32_t *plan_out);
 
+/* The launch plan of the prefill GEMM on CTA pairs: plan_out[0..7] = {tokens per tile, CTA pairs along K, clusters,
+ * tiles, decoded 64-wide stages, accumulator sets, 0, 0}; without a CUDA device for a B200.  Status 2 where that kernel
+ * does not take the shape. */
+int32_t tb200_gguf_gemm_plan(int32_t format, int64_t m, int64_t n, int64_t k, int32_t *plan_out);
+
 /* A schedule: the launch choices of the pipelined kernels that a caller may pin; a zero field means
  * "let the library derive it".  This is the counterpart of the reference's schedule dictionaries and
  * their legality predicate (src/tensor/compiler/cuda/schedules.py:3-52) for kernels that are written by

@@ -243,6 +243,25 @@ int32_t tb200_gguf_gemv_plan(int32_t format, int64_t m, int64_t n, int64_t k, in
   return TENSOR_OK;
 }
 
+int32_t tb200_gguf_gemm_plan(int32_t format, int64_t m, int64_t n, int64_t k, int32_t* plan_out) {
+  if (!plan_out) return TENSOR_ERROR_ARGUMENT;
+  for (int i = 0; i < 8; ++i) plan_out[i] = 0;
+  DeviceInfo b200;  // without a device, plan for a B200
+  b200.ordinal = 0;
+  b200.sm_count = 148;
+  b200.max_smem_optin = 232448;
+  b200.cc_major = 10;
+  cudaError_t e;
+  const DeviceInfo* dev = device_info(&e);
+  if (!dev) {
+    cudaGetLastError();
+    dev = &b200;
+  }
+  if (!gemm_pair_supported(format, m, n, k, *dev)) return TENSOR_ERROR_ARGUMENT;
+  gemm_pair_plan(format, m, n, k, *dev, plan_out);
+  return TENSOR_OK;
+}
+
 int32_t tb200_gguf_gemv_launch_config(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k,
                                       int64_t scratch_bytes, int32_t* out32) {
   if (!out32) return TENSOR_ERROR_ARGUMENT;

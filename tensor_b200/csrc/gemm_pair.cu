@@ -830,6 +830,10 @@ int resident_clusters(int splits, const DeviceInfo& dev) {
   return count;
 }
 
+// Two accumulator sets where four decoded stages fit beside them in tensor memory, eight stages where they do (log2).
+int accumulator_sets(int tokens) { return tokens <= 192 ? 2 : 1; }
+int decoded_log(int tokens) { return accumulator_sets(tokens) * tokens <= 256 ? 3 : 2; }
+
 struct PairPlan {
   int tokens, splits, clusters, tiles, token_tiles;
 };
@@ -840,11 +844,17 @@ struct PairPlan {
 // for Q4_K, 680 / 770 / 600 for Q6_K); above T = 192 one accumulator set leaves the epilogue exposed.  A tile adds its fill
 // and drain, a K split the exchange of accumulators.  Tiles go out in rounds of as many clusters as the device holds,
 // so a narrower T pays where it fills the last round better.
+//
+// A decode group takes every fourth k-block of a tile and begins the next tile where it left off, so that its k-blocks are
+// up to 4 + r apart where r = k-blocks of a tile mod 4.  It waits for a decoded stage by the parity of the stage's laps,
+// which says nothing of a stage a whole lap behind: with four stages (T = 160, 192) and r > 0 the group could write a
+// stage that has not been read yet.  Such K take a T with eight stages there, unless a cluster has one tile only.
 template <int FMT>
 PairPlan plan_pair(long long m, long long n, long long k, const DeviceInfo& dev) {
   const int decode = FMT == kQ4_K ? 500 : FMT == kQ6_K ? 650 : FMT == kQ8_0 ? 540 : 520;
   const long long row_tiles = (n + kPairRows - 1) / kPairRows;
   const int chunks = (int)((k + kChunkK - 1) / kChunkK);
+  const bool every_fourth = (k + kBlockK - 1) / kBlockK % 4 == 0;
   PairPlan best{};
   double best_cost = 1e300;
   for (int t = 32; t <= kMaxTokens; t += 32) {
@@ -855,6 +865,7 @@ PairPlan plan_pair(long long m, long long n, long long k, const DeviceInfo& dev)
     for (int s = 1; s <= 4; s *= 2) {
       if (s > 1 && (s > chunks || tiles * s > dev.sm_count / 2)) break;
       const int resident = resident_clusters<FMT>(s, dev);
+      if (!every_fourth && s == 1 && tiles > resident && decoded_log(t) == 2) continue;
       const long long rounds = (tiles + resident - 1) / resident;
       const double blocks = 4.0 * ((chunks + s - 1) / s);
       const double tile_cost = blocks * per_block + (s > 1 ? 1500.0 + 12.0 * t : t > 192 ? 42.0 * t : 300.0);
@@ -897,9 +908,8 @@ cudaError_t launch_pair(const void* x, const uint8_t* w, float* out, long long m
   a.splits = plan.splits;
   a.chunks = (int)((k + kChunkK - 1) / kChunkK);
   a.tiled = a.row_bytes % 16 == 0;
-  // two accumulator sets where four decoded stages fit beside them, eight stages where they do
-  a.acc_sets = plan.tokens <= 192 ? 2 : 1;
-  a.a_log = a.acc_sets * plan.tokens <= 256 ? 3 : 2;
+  a.acc_sets = accumulator_sets(plan.tokens);
+  a.a_log = decoded_log(plan.tokens);
   a.b_bytes = plan.tokens / 2 * kBlockK * 2;
   a.pitch = a.tiled ? R::kPitch : R::kRowPitch;
   a.raw_bytes = kCtaRows * a.pitch;
@@ -940,6 +950,16 @@ bool gemm_pair_supported(int fmt, long long m, long long n, long long k, const D
   if (!valid_format(fmt) || m < 1 || n < 1 || k < block_weights(fmt) || k % block_weights(fmt)) return false;
   if (m > (1 << 24) || n > (1 << 24) || k > (1 << 24)) return false;
   return dev.max_smem_optin >= kSmemLimit;
+}
+
+void gemm_pair_plan(int fmt, long long m, long long n, long long k, const DeviceInfo& dev, int* out8) {
+  const PairPlan plan = fmt == kQ4_0   ? plan_pair<kQ4_0>(m, n, k, dev)
+                        : fmt == kQ8_0 ? plan_pair<kQ8_0>(m, n, k, dev)
+                        : fmt == kQ4_K ? plan_pair<kQ4_K>(m, n, k, dev)
+                                       : plan_pair<kQ6_K>(m, n, k, dev);
+  const int values[8] = {plan.tokens, plan.splits, plan.clusters, plan.tiles, 1 << decoded_log(plan.tokens),
+                         accumulator_sets(plan.tokens), 0, 0};
+  std::copy(values, values + 8, out8);
 }
 
 cudaError_t launch_gemm_pair(int fmt, const void* x, const uint8_t* w, float* out, long long m, long long n, long long k,

@@ -207,6 +207,8 @@ bool gemm_shape_legal(int shape, long long m, const DeviceInfo& dev);
 // The same GEMM for all four formats on pairs of CTAs (gemm_pair.cu): what the entry points run unless a schedule pins
 // one of the shapes above.
 bool gemm_pair_supported(int fmt, long long m, long long n, long long k, const DeviceInfo& dev);
+// {tokens per tile, pairs along K, clusters, tiles, decoded stages, accumulator sets, 0, 0}
+void gemm_pair_plan(int fmt, long long m, long long n, long long k, const DeviceInfo& dev, int* out8);
 cudaError_t launch_gemm_pair(int fmt, const void* x, const uint8_t* w, float* out, long long m, long long n, long long k,
                              cudaStream_t stream, const char** detail);
 

@@ -89,6 +89,16 @@ def gemv_plan(encoding, m: int, n: int, k: int, scratch_bytes: int = 1 << 40) ->
     return plan
 
 
+def gemm_plan(encoding, m: int, n: int, k: int) -> dict:
+    """The launch plan of the prefill GEMM at this shape (see ``tb200_gguf_gemm_plan``)."""
+    out = (ctypes.c_int32 * 8)()
+    status = lib().tb200_gguf_gemm_plan(get_format(encoding).type_id, m, n, k, out)
+    if status:
+        raise ValueError(f"no plan for format {encoding!r}, m={m}, n={n}, k={k}")
+    keys = ("tokens", "k_splits", "clusters", "tiles", "decoded_stages", "accumulator_sets")
+    return dict(zip(keys, (int(v) for v in out)))
+
+
 def device_status() -> int:
     """Synchronise and return the sticky device status word (0 = no bounded wait gave up)."""
     word = ctypes.c_uint32(0)

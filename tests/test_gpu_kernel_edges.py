@@ -65,7 +65,8 @@ def test_gemm_pair_edges(name, m, n, blocks):
 
 
 @pytest.mark.parametrize("name,m,n,k", [("q4_k", 600, 12300, 512), ("q6_k", 600, 12300, 768), ("q6_k", 520, 17000, 256),
-                                        ("q8_0", 700, 11000, 544), ("q4_0", 700, 11000, 352)])
+                                        ("q8_0", 700, 11000, 544), ("q4_0", 700, 11000, 352), ("q8_0", 903, 20160, 544),
+                                        ("q4_0", 494, 11583, 4288)])
 def test_gemm_pair_several_tiles_per_pair(name, m, n, k):
     """More tiles than pairs: accumulator sets, stages and raw chunks go round."""
     raw = oracle.make_weights(name, n, k, seed=3)

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import tensor_b200 as tb
-from tensor_b200 import schedule
+from tensor_b200 import ops, schedule
 
 
 def test_spaces_and_legality_need_no_gpu():
@@ -122,3 +122,19 @@ def test_plans_leave_room_for_static_shared_memory(m, n, k):
     """The kernel has a few words of static shared memory besides what a plan asks for."""
     plan = tb.gemv_plan("q4_k", m, n, k)
     assert plan["pipelined"] and plan["smem_bytes"] + 128 <= 232448
+
+
+@pytest.mark.parametrize("name", ["q8_0", "q4_0", "q4_k", "q6_k"])
+def test_gemm_plans_never_let_a_decode_group_lap_a_stage(name):
+    """A decode group's k-blocks are up to 4 + r apart across two tiles (r = k-blocks of a tile mod 4), and its wait on a
+    decoded stage can tell one lap from the next only: a plan has that many stages, or one tile per cluster."""
+    step = tb.get_format(name).weights
+    for m in (17, 130, 160, 264, 333, 700, 903, 1347, 1905):
+        for n in (256, 3605, 11000, 20160, 28672):
+            for k in (step, 352, 544, 640, 960, 2144, 4096, 5696, 12288):
+                k = -(-k // step) * step
+                plan = ops.gemm_plan(name, m, n, k)
+                blocks = -(-k // 64)
+                apart = 4 + blocks % 4 if blocks > 4 else 4
+                assert plan["tiles"] <= plan["clusters"] or plan["decoded_stages"] >= apart, (m, n, k, plan)
+                assert plan["accumulator_sets"] * plan["tokens"] + 32 * plan["decoded_stages"] <= 512
