@@ -17,6 +17,7 @@
 //   warp 2       raw weight producer: 128 rows x 256 weights per stage, one tiled TMA copy where the row stride is a
 //                multiple of 16 bytes, else (with warp 3) asynchronous copies of the 16-byte granules around a row's bytes
 //   warps 4..7   epilogue: tcgen05.ld of one accumulator set while the MMAs fill the other (T <= 192: two sets)
+//                (Q8_0, Q4_0: with warps 24..27, the products of every two k-blocks; see kFp32Sums)
 //   warps 8..23  decode: four groups of four warps; group j decodes k-block 4 c + j (64 k) of raw chunk c, a thread
 //                one row: scales once per 64 weights, 16-byte shared loads without bank conflicts
 //
@@ -42,12 +43,31 @@ constexpr int kMaxAStages = 8;   // decoded k-blocks in tensor memory, 32 column
 constexpr int kMaxBStages = 16;
 constexpr int kMaxRawStages = 6;
 constexpr int kMaxTokens = 256;
-constexpr int kThreads = 24 * 32;
 constexpr int kDecodeWarp0 = 8;
-constexpr int kGroups = 5;       // of four warps that wait together: four that decode, one that drains
+constexpr int kDecodeWarps = 16;
+constexpr int kGroups = 6;       // of four warps that wait together: four that decode, up to two that drain
+// The 32-weight formats: the tensor cores add up one k-block only, eight drain warps the k-blocks, in fp32 registers, and
+// every kInnerSums of them in shared memory.  Accumulating in tensor memory truncates: about 1.3e-8 of the result per 16
+// of K, 2.1e-6 against fp64 at K = 4096 and 1.6e-5 at 28672, where the fp32 sums of the SIMT kernel that these formats had
+// before are 1.1e-7 and 2.8e-7 off; so they are 1.0e-7 and 1.6e-7 off (K = 512: 8.0e-8 | SIMT 6.6e-8).
+// It costs: a drained k-block takes 710 to 750 clocks instead of 540 (waits of the issuer and the drain warps; two
+// k-blocks per wait, one at a time took 1000), and 32 sums a thread next to 16 loaded products are all that 72 registers
+// hold, so a tile has 64 tokens (96, with the drain warps given more registers: the longer code does not stay in the
+// instruction cache, 333 x 12288 x 4096 131 us).  Q8_0 333 x 12288 x 4096 takes 109 us so, 47 accumulated in tensor
+// memory, 4519 on the SIMT kernel; 64 x 4096 x 4096 20 | 17 | 283.
+template <int FMT>
+constexpr bool kFp32Sums = FMT == kQ8_0 || FMT == kQ4_0;
+constexpr int kInnerSums = 8;
+constexpr int kMaxTokensFp32 = 64;
+constexpr int kSumSets = 4;  // accumulator sets: two pairs of k-blocks
+template <int FMT>
+constexpr int max_tokens() { return kFp32Sums<FMT> ? kMaxTokensFp32 : kMaxTokens; }
+template <int FMT>
+constexpr int threads_of() { return (kDecodeWarp0 + kDecodeWarps + (kFp32Sums<FMT> ? 4 : 0)) * 32; }
 constexpr int kSmemLimit = 232448;
 constexpr int kBarrierBytes = 1024;
-constexpr int kRing = kSmemLimit - 1024 /*alignment*/ - kBarrierBytes;  // activation and raw stages
+constexpr int kRing = kSmemLimit - 1024 /*alignment*/ - kBarrierBytes;  // activation and raw stages (and sums)
+constexpr int kSumBytes = kMaxTokensFp32 * kCtaRows * 4;
 
 // Raw stages: bytes of 256 weights, shared-memory row pitch of the tiled copy and of the per-row copies (room for the
 // up to 14 bytes in front, an odd number of 16-byte granules so that eight rows hit eight bank groups), stages.
@@ -134,7 +154,24 @@ __device__ __forceinline__ uint32_t all_done(const uint32_t (&bar)[4], const uin
       : "memory");
   return ok;
 }
-__device__ __forceinline__ bool wait_all(const uint32_t (&bar)[4], const uint32_t (&parity)[4]) {
+__device__ __forceinline__ uint32_t all_done(const uint32_t (&bar)[5], const uint32_t (&parity)[5]) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q, r, s, t;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 s, [%7], %8;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 t, [%9], %10;\n\t"
+      "and.pred p, p, q;\n\tand.pred r, r, s;\n\tand.pred p, p, r;\n\tand.pred p, p, t;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar[0]), "r"(parity[0]), "r"(bar[1]), "r"(parity[1]), "r"(bar[2]), "r"(parity[2]), "r"(bar[3]), "r"(parity[3]),
+        "r"(bar[4]), "r"(parity[4])
+      : "memory");
+  return ok;
+}
+template <int N>
+__device__ __forceinline__ bool wait_all(const uint32_t (&bar)[N], const uint32_t (&parity)[N]) {
 #pragma unroll 1
   for (int i = 0; i < 16384; ++i)
     if (all_done(bar, parity)) return true;
@@ -441,7 +478,7 @@ __device__ __forceinline__ void decode_chunk_row(uint32_t row, uint32_t skew, bo
 }
 
 template <int FMT>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(threads_of<FMT>(), 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const PairArgs a) {
   using R = RawCfg<FMT>;
   extern __shared__ uint8_t smem_raw[];
@@ -455,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   uint64_t* empty_b = full_b + kMaxBStages;       // the MMAs that read them are done (both CTAs)
   uint64_t* raw_full = empty_b + kMaxBStages;     // raw chunk has landed
   uint64_t* raw_empty = raw_full + kMaxRawStages;
-  uint64_t* acc_full = raw_empty + kMaxRawStages;  // [2] an accumulator set is complete (both CTAs)
+  uint64_t* acc_full = raw_empty + kMaxRawStages;  // [2] an accumulator set (kFp32Sums: pair of sets) is complete (both CTAs)
   uint64_t* acc_empty = acc_full + 2;              // [2] both CTAs have drained it (first CTA)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
   uint32_t* late = tmem_slot + 2;  // [kGroups][2], see GroupWait
@@ -474,6 +511,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int kb0 = 4 * c0, kb1 = min(4 * c1, k_blocks), kbs = kb1 - kb0;
   const int T = a.tokens;
   const int a_mask = (1 << a.a_log) - 1;
+  constexpr int kThreads = threads_of<FMT>();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxAStages; ++s) {
@@ -490,7 +528,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       ptx::mbar_init(&acc_full[b], 1);
-      ptx::mbar_init(&acc_empty[b], 2 * 4);
+      ptx::mbar_init(&acc_empty[b], 2 * (kFp32Sums<FMT> ? 8 : 4));
     }
     for (int i = 0; i < 2 * kGroups; ++i) late[i] = 0u;
     *gave_up = 0u;
@@ -554,51 +592,94 @@ __global__ void __launch_bounds__(kThreads, 1)
       int seq = 0, s = 0, t = 0;
       uint32_t parity = 0;
       bool ok = true;
-      for (int tile = cluster; tile < a.tiles && ok; tile += clusters, ++t) {
-        const int b = a.acc_sets == 2 ? (t & 1) : 0, use = a.acc_sets == 2 ? (t >> 1) : t;
-        if (!wait_bar(&acc_empty[b], (use & 1) ^ 1)) {
-          report_timeout(0x50000u | (unsigned)t);
-          *gave_up = 1u;
-          break;
+      if constexpr (kFp32Sums<FMT>) {
+        const uint32_t ae = ptx::smem_addr(acc_empty);
+        for (int tile = cluster; tile < a.tiles && ok; tile += clusters) {
+          for (int kb = kb0; kb < kb1; kb += 2, ++t) {
+            // two k-blocks at a time (an odd last one twice), each into an accumulator set of its own
+            const int count = min(2, kb1 - kb), seq1 = seq + count - 1, pair = t & 1;
+            const int s0 = s, s1 = count == 2 ? (s + 1 == a.b_stages ? 0 : s + 1) : s;
+            const uint32_t parity1 = s1 < s0 ? parity ^ 1 : parity;
+            const int a0 = seq & a_mask, a1 = seq1 & a_mask;
+            const uint32_t bar[5] = {fb + 8u * (uint32_t)s0, fa + 8u * (uint32_t)a0, fb + 8u * (uint32_t)s1, fa + 8u * (uint32_t)a1,
+                                     ae + 8u * (uint32_t)pair};
+            const uint32_t par[5] = {parity, (uint32_t)(seq >> a.a_log) & 1u, parity1, (uint32_t)(seq1 >> a.a_log) & 1u,
+                                     ((uint32_t)(t >> 1) & 1u) ^ 1u};
+            if (!wait_all(bar, par)) {
+              report_timeout(0x20000u | (unsigned)kb);
+              *gave_up = 1u;
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+            const uint32_t d = tmem_base + (uint32_t)(2 * pair * T);
+            uint64_t b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s0 * a.b_bytes));
+#pragma unroll
+            for (int i = 0; i < kBlockK / 16; ++i)
+              umma_pair(d, tmem_a + 32u * (uint32_t)a0 + 8u * i, b_desc + 2 * i, idesc, i ? 1u : 0u);
+            commit_pair(&empty_a[a0], mask);
+            commit_pair(&empty_b[s0], mask);
+            if (count == 2) {
+              b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s1 * a.b_bytes));
+#pragma unroll
+              for (int i = 0; i < kBlockK / 16; ++i)
+                umma_pair(d + (uint32_t)T, tmem_a + 32u * (uint32_t)a1 + 8u * i, b_desc + 2 * i, idesc, i ? 1u : 0u);
+              commit_pair(&empty_a[a1], mask);
+              commit_pair(&empty_b[s1], mask);
+            }
+            commit_pair(&acc_full[pair], mask);
+            seq += count;
+            s = s1 + 1 == a.b_stages ? 0 : s1 + 1;
+            parity = s1 + 1 == a.b_stages ? parity1 ^ 1 : parity1;
+          }
         }
-        ptx::tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)(b * T);
-        for (int kb = kb0; kb < kb1; kb += 2) {
-          // two k-blocks at a time (an odd last one twice)
-          const int count = min(2, kb1 - kb), seq1 = seq + count - 1;
-          const int s0 = s, s1 = count == 2 ? (s + 1 == a.b_stages ? 0 : s + 1) : s;
-          const uint32_t parity1 = s1 < s0 ? parity ^ 1 : parity;
-          const int a0 = seq & a_mask, a1 = seq1 & a_mask;
-          const uint32_t bar[4] = {fb + 8u * (uint32_t)s0, fa + 8u * (uint32_t)a0, fb + 8u * (uint32_t)s1, fa + 8u * (uint32_t)a1};
-          const uint32_t par[4] = {parity, (uint32_t)(seq >> a.a_log) & 1u, parity1, (uint32_t)(seq1 >> a.a_log) & 1u};
-          if (!wait_all(bar, par)) {
-            report_timeout(0x20000u | (unsigned)kb);
+      } else {
+        for (int tile = cluster; tile < a.tiles && ok; tile += clusters, ++t) {
+          const int b = a.acc_sets == 2 ? (t & 1) : 0, use = a.acc_sets == 2 ? (t >> 1) : t;
+          if (!wait_bar(&acc_empty[b], (use & 1) ^ 1)) {
+            report_timeout(0x50000u | (unsigned)t);
             *gave_up = 1u;
-            ok = false;
             break;
           }
           ptx::tc_fence_after();
-          {
-            const uint64_t b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s0 * a.b_bytes));
-#pragma unroll
-            for (int i = 0; i < kBlockK / 16; ++i)
-              umma_pair(d, tmem_a + 32u * (uint32_t)a0 + 8u * i, b_desc + 2 * i, idesc, (kb > kb0 || i) ? 1u : 0u);
-            commit_pair(&empty_a[a0], mask);
-            commit_pair(&empty_b[s0], mask);
+          const uint32_t d = tmem_base + (uint32_t)(b * T);
+          for (int kb = kb0; kb < kb1; kb += 2) {
+            // two k-blocks at a time (an odd last one twice)
+            const int count = min(2, kb1 - kb), seq1 = seq + count - 1;
+            const int s0 = s, s1 = count == 2 ? (s + 1 == a.b_stages ? 0 : s + 1) : s;
+            const uint32_t parity1 = s1 < s0 ? parity ^ 1 : parity;
+            const int a0 = seq & a_mask, a1 = seq1 & a_mask;
+            const uint32_t bar[4] = {fb + 8u * (uint32_t)s0, fa + 8u * (uint32_t)a0, fb + 8u * (uint32_t)s1, fa + 8u * (uint32_t)a1};
+            const uint32_t par[4] = {parity, (uint32_t)(seq >> a.a_log) & 1u, parity1, (uint32_t)(seq1 >> a.a_log) & 1u};
+            if (!wait_all(bar, par)) {
+              report_timeout(0x20000u | (unsigned)kb);
+              *gave_up = 1u;
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+            {
+              const uint64_t b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s0 * a.b_bytes));
+  #pragma unroll
+              for (int i = 0; i < kBlockK / 16; ++i)
+                umma_pair(d, tmem_a + 32u * (uint32_t)a0 + 8u * i, b_desc + 2 * i, idesc, (kb > kb0 || i) ? 1u : 0u);
+              commit_pair(&empty_a[a0], mask);
+              commit_pair(&empty_b[s0], mask);
+            }
+            if (count == 2) {
+              const uint64_t b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s1 * a.b_bytes));
+  #pragma unroll
+              for (int i = 0; i < kBlockK / 16; ++i)
+                umma_pair(d, tmem_a + 32u * (uint32_t)a1 + 8u * i, b_desc + 2 * i, idesc, 1u);
+              commit_pair(&empty_a[a1], mask);
+              commit_pair(&empty_b[s1], mask);
+            }
+            seq += count;
+            s = s1 + 1 == a.b_stages ? 0 : s1 + 1;
+            parity = s1 + 1 == a.b_stages ? parity1 ^ 1 : parity1;
           }
-          if (count == 2) {
-            const uint64_t b_desc = smem_desc_sw128(ptx::smem_addr(b_tiles + s1 * a.b_bytes));
-#pragma unroll
-            for (int i = 0; i < kBlockK / 16; ++i)
-              umma_pair(d, tmem_a + 32u * (uint32_t)a1 + 8u * i, b_desc + 2 * i, idesc, 1u);
-            commit_pair(&empty_a[a1], mask);
-            commit_pair(&empty_b[s1], mask);
-          }
-          seq += count;
-          s = s1 + 1 == a.b_stages ? 0 : s1 + 1;
-          parity = s1 + 1 == a.b_stages ? parity1 ^ 1 : parity1;
+          commit_pair(&acc_full[b], mask);
         }
-        commit_pair(&acc_full[b], mask);
       }
     }
   } else if (warp == 2 || (warp == 3 && !a.tiled)) {
@@ -654,7 +735,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-  } else if (warp >= kDecodeWarp0) {
+  } else if (warp >= kDecodeWarp0 && warp < kDecodeWarp0 + kDecodeWarps) {
     // ---------------- decode ----------------
     const int j = (warp - kDecodeWarp0) >> 2;                     // k-block of every chunk
     const int r = (warp & 3) * 32 + lane;                         // row of this CTA's half of the tile = TMEM lane
@@ -705,7 +786,86 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (lane == 0) arrive_remote(full_leader + 8u * (uint32_t)sa);
       }
     }
-  } else if (warp >= 4 && a.splits == 1) {
+  } else if (kFp32Sums<FMT> && warp >= 4) {
+    // ---------------- drain: two k-blocks' products at a time, half of the token columns a group of four warps ----------
+    ptx::grid_dependency_wait();  // the kernel before may still read or write the output
+    const int quarter = warp & 3, id = warp < kDecodeWarp0 ? 4 : 5, col0 = id == 4 ? 0 : T / 2;
+    GroupWait group{ptx::smem_addr(late + 2 * id), id};
+    const uint32_t products = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)col0;
+    const uint32_t sums = ptx::smem_addr(smem) + (uint32_t)(kRing - kSumBytes + (col0 * kCtaRows + quarter * 32 + lane) * 4);
+    const uint32_t release = map_rank(ptx::smem_addr(acc_empty), leader);
+    constexpr int kParts = max_tokens<FMT>() / 32;
+    int t = 0;
+    bool ok = true;
+    for (int tile = cluster; tile < a.tiles && ok; tile += clusters) {
+      const int n = (tile / a.token_tiles) * kPairRows + (int)half * kCtaRows + quarter * 32 + lane;
+      const int tok = (tile % a.token_tiles) * T + col0;
+      const int cols = min(T / 2, a.m - tok);  // (none left: these warps keep the others company)
+      float sum[kParts][16];
+      for (int i = 0; i < kbs; i += 2, ++t) {
+        const int pair = t & 1;
+        if (!group.one(&acc_full[pair], (uint32_t)(t >> 1) & 1u)) {
+          report_timeout(0x40000u);
+          *gave_up = 1u;
+          ok = false;
+          break;
+        }
+        ptx::tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (i + h == kbs) break;
+          const bool fresh = h == 0 && i % kInnerSums == 0;
+#pragma unroll
+          for (int c = 0; c < kParts; ++c)
+            if (16 * c < cols) {
+              uint32_t p[16];
+              tmem_ld_16(products + (uint32_t)((2 * pair + h) * T + 16 * c), p);
+              ptx::tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) sum[c][j] = (fresh ? 0.f : sum[c][j]) + __uint_as_float(p[j]);
+            }
+        }
+        ptx::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) arrive_remote(release + 8u * (uint32_t)pair);
+        if (i + 2 < kbs && (i + 2) % kInnerSums) continue;
+#pragma unroll
+        for (int c = 0; c < kParts; ++c)
+          if (16 * c < cols) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const uint32_t at = sums + (uint32_t)((16 * c + j) * kCtaRows * 4);
+              if (i >= kInnerSums) {
+                float before;
+                asm volatile("ld.shared.f32 %0, [%1];" : "=f"(before) : "r"(at));
+                sum[c][j] += before;
+              }
+              if (i + 2 < kbs) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(sum[c][j]) : "memory");
+            }
+          }
+      }
+      if (!ok) break;
+      if (a.splits > 1) {
+        // into the stages, which no MMA reads any more
+        float* part = reinterpret_cast<float*>(smem) + col0 * kCtaRows + quarter * 32 + lane;  // [tokens][128 rows]
+#pragma unroll
+        for (int c = 0; c < kParts; ++c)
+          if (16 * c < cols)
+#pragma unroll
+            for (int j = 0; j < 16; ++j) part[(16 * c + j) * kCtaRows] = sum[c][j];
+      } else if (n < a.n) {
+        float* o = a.out + (long long)tok * a.n + n;
+#pragma unroll
+        for (int c = 0; c < kParts; ++c)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            if (16 * c + j < cols) *o = sum[c][j];
+            o += a.n;
+            asm volatile("" : "+l"(o));  // (else the compiler keeps 32 addresses in registers through the loop above)
+          }
+      }
+    }
+  } else if (!kFp32Sums<FMT> && warp >= 4 && a.splits == 1) {
     // ---------------- epilogue: the accumulators of one tile while the next one's are being filled ----------------
     ptx::grid_dependency_wait();  // the kernel before may still read or write the output
     const int quarter = warp & 3;
@@ -751,7 +911,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int tok0 = (tile % a.token_tiles) * T, tok_end = min(T, a.m - tok0);
     float* part = reinterpret_cast<float*>(smem);  // [tokens][128 rows]
     __syncwarp();
-    if (warp >= 4 && warp < 8) {
+    if (!kFp32Sums<FMT> && warp >= 4 && warp < 8) {
       ptx::grid_dependency_wait();
       const int quarter = warp & 3;
       if (!GroupWait{ptx::smem_addr(late + 2 * 4), 4}.one(&acc_full[0], 0)) {
@@ -817,7 +977,7 @@ int resident_clusters(int splits, const DeviceInfo& dev) {
   attr[0].val.clusterDim.x = 2 * splits;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3((unsigned)(dev.sm_count / (2 * splits) * 2 * splits));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads_of<FMT>());
   cfg.dynamicSmemBytes = kSmemLimit;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
@@ -830,9 +990,10 @@ int resident_clusters(int splits, const DeviceInfo& dev) {
   return count;
 }
 
-// Two accumulator sets where four decoded stages fit beside them in tensor memory, eight stages where they do (log2).
-int accumulator_sets(int tokens) { return tokens <= 192 ? 2 : 1; }
-int decoded_log(int tokens) { return accumulator_sets(tokens) * tokens <= 256 ? 3 : 2; }
+// Two accumulator sets (four of 64 columns with fp32 sums) where four decoded stages fit beside them in tensor memory,
+// eight stages where they do (log2).
+int accumulator_sets(int fmt, int tokens) { return fmt == kQ8_0 || fmt == kQ4_0 ? kSumSets : tokens <= 192 ? 2 : 1; }
+int decoded_log(int fmt, int tokens) { return accumulator_sets(fmt, tokens) * tokens <= 256 ? 3 : 2; }
 
 struct PairPlan {
   int tokens, splits, clusters, tiles, token_tiles;
@@ -841,7 +1002,7 @@ struct PairPlan {
 // Tokens per tile and pairs along K by a cost model in SM clocks.  A k-block of 64 costs its MMAs (2 T clocks) or its
 // decode (128 rows x 64 weights by 16 warps, each with its waits), whichever is longer, and a little of the other
 // (measured at N = 12288, K = 4096, M = 2048: clocks per k-block at T = 128 / 192 / 256 are 550 / 620 / 515 + epilogue
-// for Q4_K, 680 / 770 / 600 for Q6_K); above T = 192 one accumulator set leaves the epilogue exposed.  A tile adds its fill
+// for Q4_K, 680 / 770 / 600 for Q6_K; for the formats with fp32 sums what the drain costs is in it); above T = 192 one accumulator set leaves the epilogue exposed.  A tile adds its fill
 // and drain, a K split the exchange of accumulators.  Tiles go out in rounds of as many clusters as the device holds,
 // so a narrower T pays where it fills the last round better.
 //
@@ -851,13 +1012,13 @@ struct PairPlan {
 // stage that has not been read yet.  Such K take a T with eight stages there, unless a cluster has one tile only.
 template <int FMT>
 PairPlan plan_pair(long long m, long long n, long long k, const DeviceInfo& dev) {
-  const int decode = FMT == kQ4_K ? 500 : FMT == kQ6_K ? 650 : FMT == kQ8_0 ? 540 : 520;
+  const int decode = FMT == kQ4_K ? 500 : FMT == kQ6_K ? 650 : FMT == kQ8_0 ? 730 : 710;
   const long long row_tiles = (n + kPairRows - 1) / kPairRows;
   const int chunks = (int)((k + kChunkK - 1) / kChunkK);
   const bool every_fourth = (k + kBlockK - 1) / kBlockK % 4 == 0;
   PairPlan best{};
   double best_cost = 1e300;
-  for (int t = 32; t <= kMaxTokens; t += 32) {
+  for (int t = 32; t <= max_tokens<FMT>(); t += 32) {
     if (t > 32 && t - 32 >= m) break;
     const long long token_tiles = (m + t - 1) / t, tiles = token_tiles * row_tiles;
     if (tiles > 0x3fffffff) continue;
@@ -865,7 +1026,7 @@ PairPlan plan_pair(long long m, long long n, long long k, const DeviceInfo& dev)
     for (int s = 1; s <= 4; s *= 2) {
       if (s > 1 && (s > chunks || tiles * s > dev.sm_count / 2)) break;
       const int resident = resident_clusters<FMT>(s, dev);
-      if (!every_fourth && s == 1 && tiles > resident && decoded_log(t) == 2) continue;
+      if (!every_fourth && s == 1 && tiles > resident && decoded_log(FMT, t) == 2) continue;
       const long long rounds = (tiles + resident - 1) / resident;
       const double blocks = 4.0 * ((chunks + s - 1) / s);
       const double tile_cost = blocks * per_block + (s > 1 ? 1500.0 + 12.0 * t : t > 192 ? 42.0 * t : 300.0);
@@ -908,13 +1069,13 @@ cudaError_t launch_pair(const void* x, const uint8_t* w, float* out, long long m
   a.splits = plan.splits;
   a.chunks = (int)((k + kChunkK - 1) / kChunkK);
   a.tiled = a.row_bytes % 16 == 0;
-  a.acc_sets = accumulator_sets(plan.tokens);
-  a.a_log = decoded_log(plan.tokens);
+  a.acc_sets = accumulator_sets(FMT, plan.tokens);
+  a.a_log = decoded_log(FMT, plan.tokens);
   a.b_bytes = plan.tokens / 2 * kBlockK * 2;
   a.pitch = a.tiled ? R::kPitch : R::kRowPitch;
   a.raw_bytes = kCtaRows * a.pitch;
   a.raw_stages = R::kStages;
-  a.b_stages = std::min(kMaxBStages, (kRing - a.raw_stages * a.raw_bytes) / a.b_bytes);
+  a.b_stages = std::min(kMaxBStages, (kRing - (kFp32Sums<FMT> ? kSumBytes : 0) - a.raw_stages * a.raw_bytes) / a.b_bytes);
   alignas(64) CUtensorMap map_x, map_w{};
   // tokens past m and columns past k read as zero
   bool ok = make_tensor_map_2d(&map_x, TmaType::kBF16, x, (unsigned long long)k, (unsigned long long)m,
@@ -934,7 +1095,7 @@ cudaError_t launch_pair(const void* x, const uint8_t* w, float* out, long long m
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(plan.clusters * 2 * plan.splits));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(threads_of<FMT>());
   cfg.dynamicSmemBytes = kSmemLimit;
   cfg.stream = stream;
   cfg.attrs = attr;
@@ -957,8 +1118,8 @@ void gemm_pair_plan(int fmt, long long m, long long n, long long k, const Device
                         : fmt == kQ8_0 ? plan_pair<kQ8_0>(m, n, k, dev)
                         : fmt == kQ4_K ? plan_pair<kQ4_K>(m, n, k, dev)
                                        : plan_pair<kQ6_K>(m, n, k, dev);
-  const int values[8] = {plan.tokens, plan.splits, plan.clusters, plan.tiles, 1 << decoded_log(plan.tokens),
-                         accumulator_sets(plan.tokens), 0, 0};
+  const int values[8] = {plan.tokens, plan.splits, plan.clusters, plan.tiles, 1 << decoded_log(fmt, plan.tokens),
+                         accumulator_sets(fmt, plan.tokens), 0, 0};
   std::copy(values, values + 8, out8);
 }
 

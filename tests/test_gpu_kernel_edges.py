@@ -82,6 +82,21 @@ def test_gemm_pair_several_tiles_per_pair(name, m, n, k):
     assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("name", ["q8_0", "q4_0"])
+@pytest.mark.parametrize("m,n,k", [(17, 300, 512), (64, 129, 544), (65, 512, 4096), (130, 257, 7936), (333, 9728, 2048),
+                                   (40, 256, 28672), (100, 300, 64), (20, 100, 32)])
+def test_gemm_of_32_weight_blocks_sums_in_fp32(name, m, n, k):
+    """These formats' prompts are added up outside the tensor cores, which truncate when they accumulate."""
+    wd = to_dev(oracle.make_weights(name, n, k, seed=k))
+    x = to_dev(oracle.make_activations(m, k, seed=m, dtype="bf16"), torch.bfloat16)
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gemm(x, wd, name, n, k, out=out)
+    want = x.double() @ tb.dequantize(wd, name, n, k).to(torch.bfloat16).double().t()
+    # four truncating steps of at most 2^-24 = 6e-8 of the sum each, and fp32 additions of 8 and of up to 56 such sums
+    # (a few 2^-24, random); accumulated over all of K in the tensor cores the error is 1e-6 at K = 2048
+    assert float((out.double() - want).norm() / want.norm()) < 3e-7
+
+
 @pytest.mark.parametrize("m,n,k", [(9, 777, 4352), (3, 257, 18944), (15, 129, 12288)])
 def test_split_gemv_with_odd_row_counts(m, n, k):
     """K split over CTAs with an odd number of partial sums: what lies behind them in the scratch stays aligned."""
