@@ -344,7 +344,7 @@ struct LaneRows {
   int valid;          // 32-weight blocks of the slice that exist
 };
 
-template <int FMT, int NT>
+template <int FMT, int XT, int NT>
 __device__ __forceinline__ void tile_item(const Frag<NT>& f, uint32_t stage, const LaneRows& ln, int tig, float (&acc)[NT][4]) {
   const float zero[4] = {0.f, 0.f, 0.f, 0.f};
   const uint32_t rA = stage + ln.row[0], rB = stage + ln.row[1];
@@ -366,8 +366,9 @@ __device__ __forceinline__ void tile_item(const Frag<NT>& f, uint32_t stage, con
       s_hi[r] = hmul2(sc1, kSixteenth);
       o_hi[r] = hmul2(sc1, kMinus64);
     }
-    // products scale * nibble, in two chains where only one column tile gives the tensor pipe something to overlap
-    constexpr int kChains = NT == 1 ? 2 : 1;
+    // products scale * nibble, in two chains where only one column tile gives the tensor pipe something to overlap, and
+    // for fp32 activations: a chain truncates at every MMA (16 x 4096 x 4096: 3.3e-7 off fp64 in one chain)
+    constexpr int kChains = NT == 1 || XT == kF32 ? 2 : 1;
     float c[kChains][NT][4];
 #pragma unroll
     for (int h = 0; h < kChains; ++h)
@@ -665,8 +666,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_frag_kernel(const FragArgs a
     for (int o = lane + 32 * share; o < slot_quads; o += 32 * owners) {
       const int col = o >> 2, r = 4 * (o & 3);
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      // (the small parts of fp32 activations first: added to the sum of the large ones each would cost it a rounding)
 #pragma unroll
-      for (int p = 0; p < kParts; ++p) {
+      for (int p = kParts - 1; p >= 0; --p) {
         uint32_t at = first + (uint32_t)b * red_bytes + (uint32_t)((col * kParts + p) * kColPitch + r) * 4;
 #pragma unroll 4
         for (int wi = 0; wi < row_warps; ++wi, at += kRed * 4) {
@@ -692,7 +694,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_frag_kernel(const FragArgs a
     const bool has_tile = live && tile < a.row_tiles;
     if (has_tile) {
       float acc[NT][4];
-      tile_item<FMT, NT>(f, stage, ln, tig, acc);
+      tile_item<FMT, XT, NT>(f, stage, ln, tig, acc);
       if (use > 0 && ok && !ptx::mbar_wait(&empty[buf], (use - 1) & 1)) {
         report_timeout(0xB0000u);
         ok = false;

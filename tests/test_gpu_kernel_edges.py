@@ -161,6 +161,20 @@ def test_gemv_frag_q4k_small_f16_activations(m, k, exponent):
     assert float((out.double() - want).norm() / want.norm()) < 2e-5
 
 
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("m,n,k", [(1, 4112, 4096), (5, 1024, 4096), (16, 512, 4096), (3, 512, 12288)])
+def test_gemv_frag_f32_sums_like_fp32_arithmetic(name, m, n, k):
+    wd = to_dev(oracle.make_weights(name, n, k, seed=m))
+    x = torch.randn((m, k), device=dev(), generator=torch.Generator(device=dev()).manual_seed(k))
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gguf(m, n, k, name, x_dtype="float32").launch(x, wd, out)
+    want = x.double() @ tb.dequantize(wd, name, n, k).double().t()
+    # fp32 additions of 8 scale groups (16 for Q6_K) and of 16 slices, each about 2.4e-8 of the running sum: 2.4e-8
+    # sqrt(8 / 2 + 16 / 2) = 8e-8, and what an MMA truncates below that; Q4_K has two chains of eight MMAs a slice, which
+    # truncate 1.3e-8 each at most
+    assert float((out.double() - want).norm() / want.norm()) < (2.6e-7 if name == "q4_k" else 1.3e-7)
+
+
 @pytest.mark.parametrize("name", ["q8_0", "q4_0", "q6_k"])
 def test_gemv_frag_special_values(name):
     """Rows with an infinity or a NaN stay with themselves; zero and tiny rows keep their scale."""
