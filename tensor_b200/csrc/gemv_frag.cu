@@ -155,6 +155,7 @@ struct Frag {
   uint32_t b[16][NT][2];
   uint32_t bm[NT][2];  // Q4_K: group sums / 64 as high and low fp16 parts
   float u[NT][2];      // factors that undo the scaling of columns 2 tig and 2 tig + 1
+  bool non_finite;     // Q4_K: some activation of the warp's slice is an infinity or a NaN
 };
 
 __device__ __forceinline__ float scale_for(uint32_t exponent) {  // largest magnitude -> [2^14, 2^15)
@@ -169,6 +170,7 @@ template <int FMT, int XT, int NT>
 __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, int sb, bool live, int gid, int tig, uint32_t spare) {
   constexpr int kParts = XT == kF32 ? 3 : 1;
   const int rest = a.k - sb * 256;  // elements of the slice that exist
+  f.non_finite = false;
   if constexpr (XT != kF32) {
     // Whole rows of the slice (512 bytes, a warp's 16-byte loads) go through shared memory, four at a time, and come
     // back in fragment order: loaded in that order from global memory, an instruction would touch a line per lane.
@@ -232,6 +234,7 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
           for (int i = 0; i < 4; ++i) {
             const uint32_t mag = q[i] & 0x7FFFFFFFu;
             if (mag < 0x7F800000u) mx = max(mx, mag);
+            else f.non_finite = true;
           }
         }
       }
@@ -277,6 +280,7 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
             asm("max.u16x2 %0, %0, %1;" : "+r"(both) : "r"(f.b[s][t][j] & 0x7FFF7FFFu));
         uint32_t mx = max(both & 0xFFFFu, both >> 16);
         if (__any_sync(0xffffffffu, mx >= kNonFinite)) {  // the scale follows the finite values
+          f.non_finite = true;
           mx = 0;
 #pragma unroll
           for (int s = 0; s < 16; ++s)
@@ -316,7 +320,7 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
     if constexpr (FMT == kQ4_K) {
       // group sums by MMA: row i of A is one where lane i of a column feeds it, so that row i of D is the sum over lane
       // i's elements; lane (column, i) then fetches its own from the lane that holds it (an infinity or a NaN reaches
-      // every group of its column, whose result is NaN anyway)
+      // every group of its column: see non_finite_sum)
       const uint32_t ones = gid == tig ? 0x3C003C00u : 0u;
       float hi[2], lo[2];
 #pragma unroll
@@ -333,6 +337,27 @@ __device__ __forceinline__ void load_fragments(Frag<NT>& f, const FragArgs& a, i
       f.bm[t][1] = pack_f16(lo[0], lo[1]);
     }
   }
+  if constexpr (FMT == kQ4_K) f.non_finite = __any_sync(0xffffffffu, f.non_finite);
+}
+
+// What a Q4_K block and the slice of one activation row come to where the slice holds an infinity or a NaN (`sum`: where it
+// does not).  The kernel multiplies quants and minimums apart, which makes inf - inf of an infinity; the product with the
+// decoded weight is an infinity of its sign.  Only terms that are not finite count.
+template <int XT>
+__device__ __noinline__ float non_finite_sum(float sum, const uint8_t* block, const void* x, long long at) {
+  bool found = false;
+#pragma unroll 1
+  for (int e = 0; e < 256; ++e) {
+    float v;
+    if constexpr (XT == kF32) v = static_cast<const float*>(x)[at + e];
+    else if constexpr (XT == kBF16) v = __bfloat162float(static_cast<const __nv_bfloat16*>(x)[at + e]);
+    else v = __half2float(static_cast<const __half*>(x)[at + e]);
+    if ((__float_as_uint(v) & 0x7F800000u) == 0x7F800000u) {
+      sum = (found ? sum : 0.f) + decode_one<kQ4_K>(block, e) * v;
+      found = true;
+    }
+  }
+  return sum;
 }
 
 // What a lane needs to know about its two rows (gid and gid + 8) of a staged tile.
@@ -695,6 +720,19 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_frag_kernel(const FragArgs a
     if (has_tile) {
       float acc[NT][4];
       tile_item<FMT, XT, NT>(f, stage, ln, tig, acc);
+      if constexpr (FMT == kQ4_K)
+        if (f.non_finite) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int col = 8 * t + 2 * tig + (j & 1), row = tile * kRows + gid + 8 * (j >> 1);
+              const bool exists = row < (tile >= second_tile ? a.n : a.n1);
+              if (col % kParts == 0 && col / kParts < a.m && exists)
+                acc[t][j] = non_finite_sum<XT>(acc[t][j], smem + (stage - ptx::smem_addr(smem)) + ln.row[j >> 1], a.x,
+                                               (long long)(col / kParts) * a.k + sb * 256);
+            }
+        }
       if (use > 0 && ok && !ptx::mbar_wait(&empty[buf], (use - 1) & 1)) {
         report_timeout(0xB0000u);
         ok = false;

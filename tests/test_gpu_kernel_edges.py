@@ -175,22 +175,35 @@ def test_gemv_frag_f32_sums_like_fp32_arithmetic(name, m, n, k):
     assert float((out.double() - want).norm() / want.norm()) < (2.6e-7 if name == "q4_k" else 1.3e-7)
 
 
-@pytest.mark.parametrize("name", ["q8_0", "q4_0", "q6_k"])
-def test_gemv_frag_special_values(name):
-    """Rows with an infinity or a NaN stay with themselves; zero and tiny rows keep their scale."""
-    n, k = 40, 512
+@pytest.mark.parametrize("x", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("name,m,k", [("q8_0", 5, 512), ("q4_0", 5, 512), ("q6_k", 5, 512), ("q4_k", 5, 4096), ("q4_k", 12, 4608)])
+def test_gemv_frag_special_values(name, m, k, x):
+    """Rows with an infinity or a NaN stay with themselves and are what the decoded weights make of them; zero and tiny
+    rows keep their scale."""
+    n = 2200 if m > 8 else 40
     wd = to_dev(oracle.make_weights(name, n, k, seed=5))
-    x = torch.randn(5, k, device=dev(), generator=torch.Generator(device=dev()).manual_seed(1)).to(torch.bfloat16)
-    x[0] = 0
-    x[1] *= 2.0 ** -100
-    x[2, 7] = float("nan")
-    x[3, 9] = float("inf")
-    out = torch.empty((5, n), device=dev())
-    tb.gguf(5, n, k, name).launch(x, wd, out)
-    want = x.double() @ tb.dequantize(wd, name, n, k).double().t()
-    assert torch.all(out[0] == 0) and torch.isnan(out[2]).all() and not torch.isfinite(out[3]).any()
-    for row in (1, 4):
-        assert float((out[row].double() - want[row]).norm() / want[row].norm()) < 1e-5
+    dtype = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[x]
+    xd = torch.randn(m, k, device=dev(), generator=torch.Generator(device=dev()).manual_seed(1))
+    xd[0] = 0
+    xd[1] *= 2.0 ** (-14 if x == "f16" else -100)
+    xd[2, 7] = float("nan")
+    xd[3, 9] = float("inf")
+    xd[m - 1, 300] = float("-inf")
+    if m > 8:
+        xd[7, 4500], xd[7, 4501] = float("inf"), float("inf")
+    xd = xd.to(dtype)
+    out = torch.empty((m, n), device=dev())
+    tb.gguf(m, n, k, name, x_dtype=dtype).launch(xd, wd, out)
+    weight = tb.dequantize(wd, name, n, k).double()
+    want = xd.double() @ weight.t()
+    assert torch.all(out[0] == 0) and torch.isnan(out[2]).all()
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(out), torch.isnan(want)) and torch.equal(torch.isfinite(out), finite)
+    assert torch.equal(torch.where(torch.isinf(out), out.sign(), 0 * out.nan_to_num()).double(),
+                       torch.where(torch.isinf(want), want.sign(), 0 * want.nan_to_num()))
+    for row in range(m):
+        if finite[row].all() and row:
+            assert float((out[row].double() - want[row]).norm() / want[row].norm()) < (2e-5 if name == "q4_k" else 1e-5)
 
 
 @pytest.mark.parametrize("name,k", [("q6_k", 768), ("q8_0", 4128), ("q4_0", 992), ("q4_k", 4096)])
