@@ -126,6 +126,10 @@ int64_t tb200_gguf_gemv_scratch_bytes(int32_t format, int64_t m, int64_t n, int6
 int32_t tb200_gguf_gemv_plan(int32_t format, int64_t m, int64_t n, int64_t k, int64_t scratch_bytes,
                              int32_t *plan_out);
 
+/* 1 where the default entry points run a GEMV with one destination and no peers on the kernel that keeps the activations
+ * in registers, as shapes and recorded schedules stand now; 0 elsewhere.  (Lists keep Q4_K items on the pipelined kernel.) */
+int32_t tb200_gguf_gemv_on_registers(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k);
+
 /* The launch plan of the prefill GEMM on CTA pairs: plan_out[0..7] = {tokens per tile, CTA pairs along K, clusters,
  * tiles, decoded 64-wide stages, accumulator sets, 0, 0}; without a CUDA device for a B200.  Status 2 where that kernel
  * does not take the shape. */
@@ -152,6 +156,8 @@ int32_t tb200_gguf_schedule_legal(int32_t op, int32_t format, int64_t m, int64_t
 int32_t tb200_gguf_schedule_record(int32_t op, int32_t format, int64_t m, int64_t n, int64_t k,
                                    const TB200Schedule *schedule);
 void tb200_gguf_schedule_clear(void);
+/* Whether a schedule that pins something is recorded for the shape; it is copied to `schedule` (zeros where none is). */
+int32_t tb200_gguf_schedule_recorded(int32_t op, int32_t format, int64_t m, int64_t n, int64_t k, TB200Schedule *schedule);
 /* The pipelined GEMV / the tcgen05 GEMM with a pinned schedule; status 2 if it is not legal at the shape. */
 int32_t tb200_gguf_gemv_scheduled(int32_t format, int32_t x_dtype, const void *x, const void *w, float *out,
                                   int64_t m, int64_t n, int64_t k, void *scratch, int64_t scratch_bytes,

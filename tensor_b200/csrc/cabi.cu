@@ -72,7 +72,8 @@ std::vector<ScheduleEntry> g_schedules;  // entries are never moved once handed 
 const Schedule* lookup_schedule(int op, int fmt, long long m, long long n, long long k) {
   std::lock_guard<std::mutex> guard(g_schedule_lock);
   for (const ScheduleEntry& e : g_schedules)
-    if (e.op == op && e.fmt == fmt && e.m == m && e.n == n && e.k == k) return &e.schedule;
+    if (e.op == op && e.fmt == fmt && e.m == m && e.n == n && e.k == k)
+      return e.schedule.pins_nothing() ? nullptr : &e.schedule;  // (an entry that was cleared, or recorded empty)
   return nullptr;
 }
 void record_schedule(int op, int fmt, long long m, long long n, long long k, const Schedule& s) {
@@ -355,6 +356,13 @@ bool use_frag(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k, 
   return !lookup_schedule(kOpGemv, format, m, n, k);  // a schedule recorded for the shape names the kernel it was searched on
 }
 
+}  // namespace
+
+extern "C" int32_t tb200_gguf_gemv_on_registers(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k) {
+  return use_frag(format, x_dtype, m, n, k, TB200_VARIANT_AUTO, 1, nullptr, nullptr) ? 1 : 0;
+}
+
+namespace {
 // Shared by the plain and the sharded entry points: `out` says where the [m, n] result goes.
 int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* w, const OutSpec& out, int64_t m,
                     int64_t n, int64_t k, void* scratch, int64_t scratch_bytes, int32_t variant, void* stream,
@@ -863,6 +871,21 @@ int32_t tb200_gguf_schedule_record(int32_t op, int32_t format, int64_t m, int64_
   if ((op != TB200_OP_GEMV && op != TB200_OP_GEMM) || !valid_format(format)) return TENSOR_ERROR_ARGUMENT;
   record_schedule(op, format, m, n, k, to_schedule(schedule));
   return TENSOR_OK;
+}
+
+int32_t tb200_gguf_schedule_recorded(int32_t op, int32_t format, int64_t m, int64_t n, int64_t k, TB200Schedule* schedule) {
+  const Schedule* s = lookup_schedule(op, format, m, n, k);
+  if (schedule) {
+    *schedule = TB200Schedule{};
+    if (s) {
+      schedule->k_splits = s->k_splits;
+      schedule->ctas_per_sm = s->ctas_per_sm;
+      schedule->convert_ahead = s->convert_ahead;
+      schedule->overlap = s->overlap;
+      schedule->gemm_shape = s->gemm_shape;
+    }
+  }
+  return s ? 1 : 0;
 }
 
 void tb200_gguf_schedule_clear(void) { clear_schedules(); }

@@ -69,6 +69,7 @@ struct Schedule {
   int convert_ahead = 0;  // GEMV, m > 1: 1 = activations converted by a kernel ahead of the GEMV, 2 = by every CTA
   int overlap = 0;        // 1 = launch with programmatic stream serialization (default), 2 = fully serialized
   int gemm_shape = 0;     // GEMM: 11, 12 or 22 = <256-token tiles per CTA, decode warp groups>
+  bool pins_nothing() const { return !k_splits && !ctas_per_sm && !convert_ahead && !overlap && !gemm_shape; }
 };
 // Schedules recorded for a shape (by a search) that the default entry points consult; nullptr if none.
 enum ScheduleOp : int { kOpGemv = 1, kOpGemm = 2 };

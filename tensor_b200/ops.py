@@ -89,6 +89,11 @@ def gemv_plan(encoding, m: int, n: int, k: int, scratch_bytes: int = 1 << 40) ->
     return plan
 
 
+def gemv_on_registers(encoding, m: int, n: int, k: int, x_dtype="bfloat16") -> bool:
+    """Whether a default GEMV of this shape runs on the kernel that keeps the activations in registers."""
+    return bool(lib().tb200_gguf_gemv_on_registers(get_format(encoding).type_id, _X_DTYPE_NAMES[x_dtype], m, n, k))
+
+
 def gemm_plan(encoding, m: int, n: int, k: int) -> dict:
     """The launch plan of the prefill GEMM at this shape (see ``tb200_gguf_gemm_plan``)."""
     out = (ctypes.c_int32 * 8)()

@@ -78,6 +78,13 @@ def record(op: str, encoding, m: int, n: int, k: int, config: dict) -> None:
         raise ValueError("cannot record a schedule for this operation or format")
 
 
+def recorded(op: str, encoding, m: int, n: int, k: int) -> dict:
+    """The schedule recorded for this exact shape (axes that pin something); ``{}`` where nothing is."""
+    s = abi.TB200Schedule()
+    lib().tb200_gguf_schedule_recorded(_OPS[op], get_format(encoding).type_id, m, n, k, ctypes.byref(s))
+    return {axis: getattr(s, axis) for axis in AXES if getattr(s, axis)}
+
+
 def clear() -> None:
     """Forget every recorded schedule (the shipped ones included): everything is derived again."""
     lib().tb200_gguf_schedule_clear()
@@ -111,13 +118,15 @@ def search(op: str, encoding, m: int, n: int, k: int, device=None, space: dict |
            repeats: int = 5, l2_bytes: int = 126 << 20, seed: int = 0) -> dict:
     """Time every legal schedule on the current GPU and return ``{"best": config, "us": ..., "rows": [...]}``.
 
-    Correctness gate first: a candidate whose output differs from the default schedule's by more than
+    The empty schedule ``{}`` stands for what the ordinary entry point does at this shape, whichever kernel that is;
+    ``best`` is ``{}`` where no pinned schedule is faster.  (One that is recorded for the shape is set aside meanwhile.)
+    Correctness gate first: a candidate whose output differs from the ordinary one's by more than
     ``tolerance`` (relative Frobenius norm) is rejected and never timed.  Timing: CUDA events around
     a CUDA graph that walks enough distinct weight copies to exceed three times the L2 cache, median of
     ``repeats`` replays (the reference conditions L2 between samples, tuning.py:15-82)."""
     import torch
 
-    from . import synth
+    from . import ops, synth
     from .ops import gemv_scratch_bytes
 
     fmt = get_format(encoding)
@@ -129,33 +138,46 @@ def search(op: str, encoding, m: int, n: int, k: int, device=None, space: dict |
     # a split finer than the default plan's needs more partial-sum space
     scratch = torch.zeros(max(need, 4096 + 64 * m * n * 4), dtype=torch.uint8, device=device) if op == "gemv" else None
     out = torch.empty((m, n), dtype=torch.float32, device=device)
-    reference = run_scheduled(op, x, ws[0], fmt, n, k, {}, torch.empty_like(out), scratch).clone()
+    pinned = recorded(op, fmt, m, n, k)
+
+    def run(w, config, stream=None):
+        if config:
+            return run_scheduled(op, x, w, fmt, n, k, config, out, scratch, stream=stream)
+        if op == "gemv":
+            return ops.gemv(x, w, fmt, n, k, out=out, scratch=scratch, stream=stream)
+        return ops.gemm(x, w, fmt, n, k, out=out, stream=stream)
+
     stream = torch.cuda.Stream(device)
     rows = []
-    for config in candidates(op, fmt, m, n, k, space):
-        try:
-            got = run_scheduled(op, x, ws[0], fmt, n, k, config, out, scratch).clone()
-        except ValueError:
-            continue  # legal on paper, refused at this scratch size
-        error = float((got - reference).norm() / reference.norm())
-        if not error <= tolerance:
-            rows.append({"config": config, "rejected": f"relative error {error:.2e}"})
-            continue
-        with torch.cuda.stream(stream):
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph, stream=stream):
-                for w in ws:
-                    run_scheduled(op, x, w, fmt, n, k, config, out, scratch, stream=stream)
-            graph.replay()
-            samples = []
-            for _ in range(repeats):
-                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-                e0.record(stream)
+    record(op, fmt, m, n, k, {})
+    try:
+        reference = run(ws[0], {}).clone()
+        for config in candidates(op, fmt, m, n, k, space):
+            try:
+                got = run(ws[0], config).clone()
+            except ValueError:
+                continue  # legal on paper, refused at this scratch size
+            error = float((got - reference).norm() / reference.norm())
+            if not error <= tolerance:
+                rows.append({"config": config, "rejected": f"relative error {error:.2e}"})
+                continue
+            with torch.cuda.stream(stream):
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=stream):
+                    for w in ws:
+                        run(w, config, stream=stream)
                 graph.replay()
-                e1.record(stream)
-                stream.synchronize()
-                samples.append(e0.elapsed_time(e1) * 1e3 / copies)
-        rows.append({"config": config, "us": statistics.median(samples), "error": error})
+                samples = []
+                for _ in range(repeats):
+                    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                    e0.record(stream)
+                    graph.replay()
+                    e1.record(stream)
+                    stream.synchronize()
+                    samples.append(e0.elapsed_time(e1) * 1e3 / copies)
+            rows.append({"config": config, "us": statistics.median(samples), "error": error})
+    finally:
+        record(op, fmt, m, n, k, pinned)
     timed = [r for r in rows if "us" in r]
     best = min(timed, key=lambda r: r["us"])
     return {"op": op, "format": fmt.name, "m": m, "n": n, "k": k, "best": best["config"], "us": best["us"],
@@ -193,4 +215,4 @@ class Profile:
 
 
 __all__ = ["AXES", "DECODE_SPACE", "PREFILL_SPACE", "Profile", "candidates", "clear", "legal", "projection_space",
-           "record", "run_scheduled", "search"]
+           "record", "recorded", "run_scheduled", "search"]

@@ -44,6 +44,27 @@ def test_recorded_schedule_becomes_the_default_plan():
     assert tb.gemv_plan(*shape) == derived
 
 
+def test_a_cleared_or_empty_schedule_leaves_the_default_kernel():
+    """A recorded schedule names the pipelined kernel; forgotten, or recorded empty, it must not keep a shape there."""
+    from tensor_b200 import _native
+
+    shape = ("q4_k", 16, 7296, 8192)
+    schedule.clear()
+    try:
+        assert ops.gemv_on_registers(*shape) and schedule.recorded("gemv", *shape) == {}
+        schedule.record("gemv", *shape, {"k_splits": 2, "ctas_per_sm": 1})
+        assert not ops.gemv_on_registers(*shape)
+        assert schedule.recorded("gemv", *shape) == {"k_splits": 2, "ctas_per_sm": 1}
+        schedule.record("gemv", *shape, {})
+        assert ops.gemv_on_registers(*shape)
+        schedule.record("gemv", *shape, {"k_splits": 2})
+        schedule.clear()
+        assert ops.gemv_on_registers(*shape) and schedule.recorded("gemv", *shape) == {}
+        assert ops.gemv_on_registers("q4_k", 16, 1792, 18944)  # shipped with one
+    finally:
+        _native._apply_shipped_schedules()
+
+
 def test_derived_plan_counts_the_latency_of_a_split():
     """Batch 1 at K = 4096: a K split balances the SMs on paper but its extra phase costs about 2 us, more than
     the whole unsplit launch takes (measured 4.4 against 11.6 us at 3072 rows): the derived plan must not split.
@@ -108,6 +129,24 @@ def test_measured_search_behind_the_parity_gate(op, name, m, n, k):
     finally:
         schedule.clear()
     assert tb.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_search_measures_against_the_ordinary_entry_point(monkeypatch):
+    """The empty schedule is what a call without one runs (here the register kernel), and what was recorded stays."""
+    shape = ("q4_k", 16, 640, 4352)
+    calls = []
+    real = ops.gemv
+    monkeypatch.setattr(ops, "gemv", lambda *a, **kw: (calls.append(ops.gemv_on_registers(*shape)), real(*a, **kw))[1])
+    schedule.record("gemv", *shape, {"k_splits": 2})
+    try:
+        result = schedule.search("gemv", *shape, repeats=2, l2_bytes=4 << 20, space={"k_splits": (1, 2)})
+        assert schedule.recorded("gemv", *shape) == {"k_splits": 2}
+    finally:
+        schedule.record("gemv", *shape, {})
+    assert calls and all(calls)
+    assert result["rows"][0]["config"] == {} and result["default_us"] == result["rows"][0]["us"]
+    assert len([r for r in result["rows"] if "us" in r]) >= 2
 
 
 @pytest.mark.parametrize("m,n,k", [(9, 777, 4352), (3, 257, 18944), (15, 129, 12288), (2, 1031, 28672)])
