@@ -234,11 +234,20 @@ def gemv_sharded(x: torch.Tensor, w: torch.Tensor, encoding, n: int, k: int, out
             max(len(pads), 1), sync, _stream_handle(device, stream))
 
 
+def _cuda_device(device) -> torch.device:
+    """``device`` with an index: a ``torch.device`` (the current one where it has none), its text, an index or ``None``."""
+    device = torch.device("cuda", device) if isinstance(device, int) else torch.device("cuda" if device is None else device)
+    if device.type != "cuda":
+        raise ValueError(f"expected a CUDA device, got {device}")
+    return device if device.index is not None else torch.device("cuda", torch.cuda.current_device())
+
+
 def peer_sync(pad_ptrs, rank: int, device: torch.device, mode: int = PEER_WAIT | PEER_SIGNAL, stream=None) -> None:
     """Enqueue one or both halves of the cross-GPU barrier (``tb200_peer_sync``) on ``stream``;
     ``pad_ptrs[i]`` is the address of rank i's signal pad as mapped in this process."""
     ptrs = [int(p) for p in pad_ptrs]
     table = (ctypes.c_void_p * max(len(ptrs), 1))(*ptrs)
+    device = _cuda_device(device)
     _invoke(lib().tb200_peer_sync, device, table, rank, len(ptrs), mode, _stream_handle(device, stream))
 
 

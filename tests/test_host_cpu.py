@@ -215,6 +215,35 @@ def test_peer_barrier_rejects_bad_ranks():
     assert lib().tb200_peer_barrier(table, 0, 2, None, ctypes.byref(err)) == 3
 
 
+@pytest.mark.parametrize("device,index", [("cuda", 3), ("cuda:0", 0), (None, 3), (3, 3), (0, 0)])
+def test_peer_sync_takes_a_device_in_every_form(monkeypatch, device, index):
+    """Without an index the current device is meant; the argument check of the call itself comes before any CUDA call."""
+    import torch
+
+    from tensor_b200 import ops
+
+    streams, entered = [], []
+
+    class Entered:
+        def __init__(self, d):
+            entered.append(torch.device(d).index)
+
+        __enter__ = __exit__ = lambda self, *a: None
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "device", Entered)
+    monkeypatch.setattr(ops, "_raw_stream", lambda i: streams.append(i) or 0)
+    forms = [device] + ([torch.device(device)] if isinstance(device, str) else [])
+    for form in forms:
+        with pytest.raises(ValueError, match="rank 5 of world 1"):
+            ops.peer_sync([64], 5, form)
+        with pytest.raises(ValueError, match="rank 5 of world 1"):
+            ops.peer_barrier([64], 5, form)
+    assert streams == [index] * 2 * len(forms) and entered == ([] if index == 3 else [0] * 2 * len(forms))
+    with pytest.raises(ValueError):
+        ops.peer_sync([64], 0, "cpu")
+
+
 def test_bump_allocator_gives_every_rank_the_same_offsets():
     from tensor_b200.peer import BumpAllocator
 
