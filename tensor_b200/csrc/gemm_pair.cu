@@ -995,6 +995,8 @@ int resident_clusters(int splits, const DeviceInfo& dev) {
 int accumulator_sets(int fmt, int tokens) { return fmt == kQ8_0 || fmt == kQ4_0 ? kSumSets : tokens <= 192 ? 2 : 1; }
 int decoded_log(int fmt, int tokens) { return accumulator_sets(fmt, tokens) * tokens <= 256 ? 3 : 2; }
 
+constexpr long long kMaxTiles = 0x3fffffff;
+
 struct PairPlan {
   int tokens, splits, clusters, tiles, token_tiles;
 };
@@ -1021,7 +1023,7 @@ PairPlan plan_pair(long long m, long long n, long long k, const DeviceInfo& dev)
   for (int t = 32; t <= max_tokens<FMT>(); t += 32) {
     if (t > 32 && t - 32 >= m) break;
     const long long token_tiles = (m + t - 1) / t, tiles = token_tiles * row_tiles;
-    if (tiles > 0x3fffffff) continue;
+    if (tiles > kMaxTiles) continue;
     const double per_block = t > 192 ? std::max(2.0 * t, decode + 50.0) : decode + 0.6 * std::max(0, 2 * t - 200);
     for (int s = 1; s <= 4; s *= 2) {
       if (s > 1 && (s > chunks || tiles * s > dev.sm_count / 2)) break;
@@ -1110,6 +1112,9 @@ TB200_DEFINE_STATUS_READER(read_gemm_pair_status)
 bool gemm_pair_supported(int fmt, long long m, long long n, long long k, const DeviceInfo& dev) {
   if (!valid_format(fmt) || m < 1 || n < 1 || k < block_weights(fmt) || k % block_weights(fmt)) return false;
   if (m > (1 << 24) || n > (1 << 24) || k > (1 << 24)) return false;
+  // (the planner has nothing to offer above so many of the largest tiles)
+  const long long tokens = fmt == kQ8_0 || fmt == kQ4_0 ? kMaxTokensFp32 : kMaxTokens;
+  if ((m + tokens - 1) / tokens * ((n + kPairRows - 1) / kPairRows) > kMaxTiles) return false;
   return dev.max_smem_optin >= kSmemLimit;
 }
 

@@ -177,3 +177,11 @@ def test_gemm_plans_never_let_a_decode_group_lap_a_stage(name):
                 apart = 4 + blocks % 4 if blocks > 4 else 4
                 assert plan["tiles"] <= plan["clusters"] or plan["decoded_stages"] >= apart, (m, n, k, plan)
                 assert plan["accumulator_sets"] * plan["tokens"] + 32 * plan["decoded_stages"] <= 512
+
+
+@pytest.mark.parametrize("name", ["q8_0", "q4_k"])
+def test_gemm_plan_of_extents_beyond_every_tile_count(name):
+    """No plan, instead of one of zero tokens a tile that a launch would divide by."""
+    with pytest.raises(ValueError):
+        ops.gemm_plan(name, 1 << 24, 1 << 24, 256)
+    assert ops.gemm_plan(name, 1 << 20, 1 << 22, 256)["tokens"] > 0
