@@ -676,7 +676,7 @@ def run_gpu(args):
                 "e2e_ms": e2e_ms, "e2e_gbps": total / (e2e_ms * 1e-3) / 1e9,
                 "launches_per_layer": 4,
                 "note": "q/k/v, o, gate/up in Q4_K (gemv_mma_kernel), down in Q6_K (batch 1: gemv_dp4a_kernel, batch 16: "
-                        "gemv_tc_kernel); the rows of q, k, v live in one 6144-row weight and those of "
+                        "gemv_frag_kernel on one GPU, gemv_tc_kernel N-sharded); the rows of q, k, v live in one 6144-row weight and those of "
                         "gate, up in one 24576-row weight (concatenated at load time), so a layer is four GEMV launches; "
                         "projections only (no attention or glue); 121.5 MB of distinct weights per layer, so every launch "
                         "streams from HBM"})

@@ -99,8 +99,8 @@ typedef struct TensorErrorV1 {
 #define TB200_VARIANT_FAST 2   /* a pipelined tensor-core kernel or an error: GEMV bulk-copy ring + mma.sync, GEMM tcgen05 */
 #define TB200_VARIANT_MMA 3    /* GEMV only: the same as FAST */
 #define TB200_VARIANT_TC 4     /* GEMV only: the persistent tcgen05 / TMEM kernel (Q4_K, Q6_K; needs scratch), or an
-                                * error.  AUTO picks it for Q6_K above one activation row only in launches that wait
-                                * for or signal peers */
+                                * error.  AUTO picks it for Q6_K above one activation row only in launches that store
+                                * into several outputs or that wait for or signal peers */
 #define TB200_VARIANT_DP4A 5   /* GEMV only, m = 1, every format: integer dot products against the activations split into
                                 * three exact 8-bit limbs (no scratch), or an error.  AUTO picks it at m = 1 for Q6_K,
                                 * Q8_0 and Q4_0 */

@@ -341,15 +341,18 @@ bool use_frag(int32_t format, int32_t x_dtype, int64_t m, int64_t n, int64_t k, 
     if (n <= (m == 1 ? 4096 : m == 2 ? 1536 : 0)) return false;
   }
   if (format == kQ4_K && x_dtype != kF32) {
-    // (a list converts the activations of all its launches ahead, which leaves its own pipeline ahead: three
-    // projections of 18944 x 3584 at batches 1, 4 and 16 take 138 us so and 154 with the batch-16 launches here)
+    // (A list converts the activations of all its launches ahead, which its own pipeline gains from: three projections of
+    // 18944 x 3584 at batches 1, 4 and 16 take 138 us so and 154 with the batch-16 launches here.  Measured on that list
+    // only; a 36-layer step at batch 16 as lists takes 3.56 ms, as plain launches 2.87.)
     if (prep_mode != kPrepNormal) return false;
-    // Q4_K's own pipeline fits two CTAs on an SM up to K = 3584, where it is ahead (12288 x 3584, batch 8 / 16: 13.5 |
-    // 11.4, 18.1 | 15.5), and one beyond.  Two column tiles (m > 8): 7296 rows, batch 16, K = 3840 13.0 | 21.1, 8192 21.2 |
-    // 26.7, 14336 35.3 | 45.4, 28160 70 | 74; not so for few rows at batches just above 8 (2048 x 4096, batch 12: 8.1 |
-    // 7.3).  One column tile: only where K fills all sixteen warps of every CTA (7296 rows, batch 8, K = 4096 9.9 | 12.1,
-    // 8192 16.3 | 21.5, 12288 22.2 | 23.0, but 7168 15.4 | 15.1, 14336 26.7 | 23.5, 18944 with fifteen and clusters of five
-    // 32.9 | 33.3, 28160 51 | 47), and with rows enough to pay for a cluster (2048 x 8192, batch 2: 8.2 | 7.4).
+    // The lines are where the measurements turn.  Up to K = 3584 Q4_K's own pipeline never splits K and is ahead (12288 x
+    // 3584, batch 8 / 16: 13.5 | 11.4, 18.1 | 15.5); at batch 16 it splits K over two or three CTAs from K = 3840 on, which
+    // adds a phase through global memory.  Two column tiles (m > 8): 7296 rows, batch 16, K = 3840 13.0 | 21.1, 8192 21.2
+    // | 26.7, 14336 35.3 | 45.4, 28160 70 | 74; not so for few rows at batches just above 8, which it does not split yet
+    // (2048 x 4096, batch 12: 8.1 | 7.3).  One column tile: only where K fills all sixteen warps of every CTA (7296 rows,
+    // batch 8, K = 4096 9.9 | 12.1, 8192 16.3 | 21.5, 12288 22.2 | 23.0, but 7168 15.4 | 15.1, 14336 26.7 | 23.5, 18944 with
+    // fifteen and clusters of five 32.9 | 33.3, 28160 51 | 47), and with rows enough to pay for a cluster (2048 x 8192,
+    // batch 2: 8.2 | 7.4).  One to six sizes stand behind each line.
     if (k <= 3584) return false;
     if (m > 8 ? m <= 12 && n <= 2048 && k <= 4096 : k % 4096 || k > 12288 || (k > 4096 && n < 4096)) return false;
   }
@@ -413,9 +416,9 @@ int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* 
                 "the integer dot-product GEMV takes m = 1 with 2-byte activations, K a multiple of 256 "
                 "(2048 for Q6_K) up to 32768 (format %d, dtype %d, m=%lld, n=%lld, k=%lld)",
                 format, x_dtype, (long long)m, (long long)n, (long long)k);
-  // The tensor-memory kernel: on request, and by default for Q6_K, which has no other pipelined GEMV
-  // (measured 1.0x .. 10x faster than the SIMT kernels there).  For Q4_K it is measured slower than the
-  // mma.sync pipeline at every batch on B200, so the default never picks it.
+  // The tensor-memory kernel: on request (FAST names it for Q6_K), and by default for Q6_K launches of 2 to 16 rows that
+  // the register kernel does not take: several destinations, or peers to wait for or signal (1.0x .. 10x faster than the
+  // SIMT kernels there).  For Q4_K it is measured slower than the mma.sync pipeline at every batch on B200.
   const bool tc_default = format == kQ6_K && (variant == TB200_VARIANT_AUTO || variant == TB200_VARIANT_FAST) &&
                           gemv_tc_supported(format, x_dtype, m, n, k);
   if (variant == TB200_VARIANT_TC || tc_default) {
@@ -436,7 +439,7 @@ int32_t gemv_common(int32_t format, int32_t x_dtype, const void* x, const void* 
       return ok(error);
     }
     if (variant == TB200_VARIANT_TC)
-    return fail(error, TENSOR_ERROR_ARGUMENT,
+      return fail(error, TENSOR_ERROR_ARGUMENT,
                 "the tensor-memory GEMV needs format 12 or 14 (K a multiple of 2048), 2-byte activations, m <= 16 and %lld bytes of scratch "
                 "(format %d, dtype %d, m=%lld, n=%lld, k=%lld, scratch %lld)",
                 need, format, x_dtype, (long long)m, (long long)n, (long long)k,

@@ -16,15 +16,16 @@
 //    weights, so the block scale d is applied once per 256 weights and the minimums are one more MMA against the group
 //    sums (kept as two fp16 parts); the other formats' centred integers, with d (and Q6_K's 8-bit scale, whose product
 //    with the quant would not fit 11 bits) applied to the fp32 accumulators of a scale group;
-//  * bf16 activations are multiplied by one power of two per (row, slice) and then fit fp16 exactly (values down to
-//    2^-29 of the largest; fp16 ones, for Q4_K, by one that keeps them exact); fp32 ones are split exactly into three
-//    fp16 parts on three columns.
+//  * bf16 activations are multiplied by one power of two per (row, slice) and then fit fp16 exactly down to 2^-29 of the
+//    slice's largest value (smaller ones are off by up to 2^-40 of it; fp16 ones, for Q4_K, by one that keeps them
+//    exact); fp32 ones are split into three fp16 parts on three columns, exactly down to 2^-15 of the largest value and
+//    to 2^-40 of it below.
 //
 // The warps of a CTA cover up to 4096 of K; a longer K is spread over the CTAs of a cluster, which add their sums through
 // distributed shared memory.  All sums are added in K order: no scratch, no atomics, the same bits on every launch.
 //
-// What bounds it is instruction issue: about 500 warp instructions per 16 x 256 weights (Q4_K, batch 8), half of the issue
-// slots used, DRAM at a fifth of its rate.  Measured (us, this kernel | the one before; graph replay over weights larger
+// What bounds it is instruction issue: 600 (Q4_K, batch 8) to 830 (Q6_K, batch 4) warp instructions per 16 x 256 weights,
+// half of the issue slots used by the four warps a scheduler that 128 registers allow, DRAM at a fifth of its rate.  Measured (us, this kernel | the one before; graph replay over weights larger
 // than the L2): Q6_K 4096 x 12288 at batch 4 / 16 19.1 | 39.7 and 26.2 | 46.5 (tensor memory), Q8_0 12288 x 4096 18.5 | 72.3
 // and 23.6 | 228, Q4_0 13.6 | 60.9 and 18.5 | 178 (SIMT), Q4_K 24576 x 4096 20.9 | 24.5 and 28.3 | 41.2 (gemv_mma.cu).
 #include <cuda_fp16.h>
@@ -821,8 +822,8 @@ int resident(int splits, const DeviceInfo& dev) {
 }
 
 // CTAs along K (a cluster) and row tiles at once.  The unit is one warp's work on 16 x 256 weights, of which an SM does one
-// after another at its own rate (about 100 clocks): a plan costs the units of its busiest SM, a meeting of the warps per
-// tile, and the exchange of a cluster (about a thousand clocks).
+// after another at its own rate (about 100 clocks): a plan costs the units of its busiest SM, what a tile costs beyond its
+// decode (three units: buffers, barriers, adding up), and the exchange of a cluster (about a thousand clocks).
 template <int FMT, int XT, int NT>
 FragPlan plan_frag(int m, int row_tiles, int nsb, const DeviceInfo& dev) {
   using C = Cfg<FMT>;
@@ -865,7 +866,8 @@ cudaError_t launch_typed(FragArgs a, cudaStream_t stream) {
   a.phase = plan.phase;
   // A cluster launch that may start while a plain one drains (or the other way round) costs about 4 us: Q4_K 24576 x 4096 and
   // 4096 x 12288 in turn at batch 8 take 45.1 us so and 37.3 with the cluster launches serialized, which is the sum of
-  // the two alone; cluster launches one after another lose 1 us each by it.
+  // the two alone; cluster launches one after another lose 1.6 us each by it (Q4_K and Q6_K 4096 x 12288 in turn: 34.7 us
+  // for the two when they may overlap, 37.9 so).
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = plan.splits > 1 ? 0 : 1;

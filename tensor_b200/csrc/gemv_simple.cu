@@ -1,7 +1,7 @@
 // SIMT fallback GEMV/GEMM: out[m, n] = x[m, k] . dequant(w[n, k])^T, one warp per weight row,
 // fp32 decode and fp32 FMA.  It accepts every shape the formats allow; the library takes it for a GEMV
-// with m > 16 or K > 32768, for small launches with fp32 activations, for launches of Q8_0 and Q4_0 that wait
-// for peers, and on request.  Contract:
+// with m > 16 or K > 32768, for small launches with fp32 activations, for batched launches of Q8_0 and Q4_0 (and fp32
+// ones) that store into several outputs or wait for or signal peers, and on request.  Contract:
 // benchmarks/kernels/showcase/triton_kernels.py:213-222 (fp32 weight x fp32 activation); with
 // weights_bf16 the decoded weight is rounded to bf16 first (the GEMM contract, :201-207).
 #include <cstdlib>

@@ -135,6 +135,28 @@ def test_gemv_frag_edges(name, m, n, blocks, x):
     assert float((out.double() - want).norm() / want.norm()) < (2e-5 if name == "q4_k" else 1e-5)
 
 
+@pytest.mark.parametrize("name,m,n,k,x", [
+    ("q8_0", 1, 31, 96, "f32"), ("q8_0", 2, 2000, 512, "f32"), ("q8_0", 1, 4097, 4096, "f32"), ("q8_0", 3, 17, 4096, "f32"),
+    ("q8_0", 1, 33, 96, "bf16"), ("q4_0", 1, 31, 96, "f32"), ("q4_0", 16, 100, 8224, "f32"), ("q4_0", 1, 40, 4128, "f16"),
+    ("q6_k", 1, 31, 256, "f32"), ("q6_k", 2, 1537, 2048, "f32"), ("q6_k", 1, 130, 12288, "f32"), ("q6_k", 1, 50, 768, "bf16"),
+    ("q4_k", 1, 31, 256, "f32"), ("q4_k", 4, 300, 18432, "f32"), ("q4_k", 9, 2100, 3840, "f16"), ("q4_k", 16, 2500, 4352, "f16"),
+    ("q4_k", 8, 513, 4096, "f16"), ("q4_k", 5, 4100, 8192, "f16"), ("q4_k", 2, 4097, 12288, "bf16"),
+    ("q4_k", 16, 20, 28672, "bf16"), ("q4_k", 16, 33, 32768, "f16"),
+])
+def test_gemv_frag_shapes_that_run_on_it(name, m, n, k, x):
+    """Of the launches that other kernels share, sizes that the default sends to the register kernel."""
+    dtype = {"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[x]
+    assert tb.ops.gemv_on_registers(name, m, n, k, dtype)
+    wd = to_dev(oracle.make_weights(name, n, k, seed=n))
+    xd = to_dev(oracle.make_activations(m, k, seed=k, dtype=x), dtype)
+    out = torch.full((m, n), float("nan"), device=dev())
+    tb.gguf(m, n, k, name, x_dtype=dtype).launch(xd, wd, out)
+    want = xd.double() @ tb.dequantize(wd, name, n, k).double().t()
+    # fp32 sums of 16-slice CTAs: 2.4e-8 sqrt(8 + 4) = 8e-8 at K = 4096, a little more per CTA of a cluster; Q4_K's chains
+    # truncate up to 16 times 1.3e-8 besides
+    assert float((out.double() - want).norm() / want.norm()) < (1e-6 if name == "q4_k" else 4e-7)
+
+
 def balanced_q4_k(n, k, seed):
     """Q4_K blocks as a quantised weight of mean zero has them: every group's minimum is 7.5 times its scale."""
     raw = oracle.make_weights("q4_k", n, k, seed=seed).reshape(-1, 144)
@@ -149,7 +171,8 @@ def balanced_q4_k(n, k, seed):
 @pytest.mark.parametrize("m,k", [(4, 4096), (16, 4096), (4, 12288), (16, 12288)])
 def test_gemv_frag_q4k_small_f16_activations(m, k, exponent):
     """The minimums' share of a result is as large as the quants': group sums keep their precision at every magnitude."""
-    n = 272
+    n = 272 if k == 4096 else 4112
+    assert tb.ops.gemv_on_registers("q4_k", m, n, k, "float16")
     wd = to_dev(balanced_q4_k(n, k, seed=k))
     gen = torch.Generator(device=dev()).manual_seed(m)
     x = (torch.randn((m, k), device=dev(), generator=gen) * 2.0 ** exponent).to(torch.float16)
@@ -192,6 +215,7 @@ def test_gemv_frag_special_values(name, m, k, x):
     if m > 8:
         xd[7, 4500], xd[7, 4501] = float("inf"), float("inf")
     xd = xd.to(dtype)
+    assert tb.ops.gemv_on_registers(name, m, n, k, dtype)
     out = torch.empty((m, n), device=dev())
     tb.gguf(m, n, k, name, x_dtype=dtype).launch(xd, wd, out)
     weight = tb.dequantize(wd, name, n, k).double()
